@@ -104,6 +104,8 @@ class BatchEmitter:
              "  extern __shared__ __align__(16) unsigned char xg_smem[];",
              "  __shared__ int64_t item_;",
              "  __shared__ int prob_;",
+             "  const xg_fp64 xg_f = xg_fp64_units();",
+             "  (void)xg_f;",
              "  const int tid = threadIdx.x + blockDim.x * threadIdx.y;",
              f"  const int HY = T * {ry}, HX = T * {rx};",
              "  const int PX = tbx + 2 * HX, PY = tby + 2 * HY;",
@@ -282,6 +284,8 @@ class BatchEmitter:
              f"int64_t total, int rot, unsigned long long* __restrict__ counter) {{",
              "  __shared__ int64_t item_;",
              "  __shared__ int prob_;",
+             "  const xg_fp64 xg_f = xg_fp64_units();",
+             "  (void)xg_f;",
              "  const int tid = threadIdx.x + blockDim.x * (threadIdx.y + blockDim.y * threadIdx.z);",
              "  // work queue: thread 0 takes the next item while the CTA works on the current one",
              "  int64_t next = 0;",

@@ -65,13 +65,17 @@ TILE_PROLOGUE = ["  const xg_tile T = xg_tile_of(p.Z, p.Y, p.X, p.tz, p.ty, p.tx
                  "  const int64_t t = T.t;",
                  "  const int z0 = T.z0, z1 = T.z1, y0 = T.y0, y1 = T.y1, x0 = T.x0, x1 = T.x1;",
                  "  const I sy = (I)p.X, sz = (I)(p.X * p.Y);",
-                 "  (void)sy; (void)sz; (void)t;"]
+                 "  const xg_fp64 xg_f = xg_fp64_units();",
+                 "  (void)sy; (void)sz; (void)t; (void)xg_f;"]
 # I is the kernel's index type: int when the grid has fewer than 2^31 cells
 CELL_LOOP = ["  for (int z = z0; z < z1; ++z)",
              "  for (int y = y0 + (int)threadIdx.y; y < y1; y += (int)blockDim.y) {",
              "    const I row_ = (I)z * sz + (I)y * sy;",
              "    for (int x = x0 + (int)threadIdx.x; x < x1; x += (int)blockDim.x) {",
              "    const I c = row_ + (I)x;"]
+
+# FP64 operations of sweeps run as fused multiply-adds (same results, faster issue: xgrid_gen.cuh)
+FMA64 = {ir.BinaryOperator.Add: "xg_dadd", ir.BinaryOperator.Sub: "xg_dsub", ir.BinaryOperator.Mul: "xg_dmul"}
 
 _INT_RANK = {"bool": 0, "int8_t": 1, "int16_t": 2, "int": 3, "int32_t": 3, "int64_t": 4}
 
@@ -210,13 +214,14 @@ class CudaGenerator:
         sub = env.substitute(e)
         if sub is not None:
             return sub
+        fma64 = getattr(env, "fma64", False)
         div = getattr(env, "div_map", {}).get(id(e))
         if div is not None:
-            return f"xg_divk((double)({self.expr(e.left, env)}), p.h.{div.name})"
+            return f"xg_divk((double)({self.expr(e.left, env)}), p.h.{div.name}, xg_f)"
         mul = getattr(env, "mul_map", {}).get(id(e))
         if mul is not None:
             h, other = mul
-            return f"xg_mulk((double)({self.expr(other, env)}), p.h.{h.name})"
+            return f"xg_mulk((double)({self.expr(other, env)}), p.h.{h.name}, xg_f)"
         if isinstance(e, ir.Constant):
             return literal(e.value)
         if isinstance(e, ir.Identifier):
@@ -242,6 +247,8 @@ class CudaGenerator:
                 base = self.expr(e.left, env)
                 t = "double" if double else "float"
                 if k == 2.0:
+                    if double and fma64:
+                        return f"xg_dsq((double)({base}), xg_f)"
                     return f"xg_sq_{'d' if double else 'f'}(({t})({base}))"
                 if k == 1.0:
                     return f"(({t})({base}))"
@@ -265,11 +272,20 @@ class CudaGenerator:
                 if soft:
                     fn = "xg_dadd_i" if e.operator is ir.BinaryOperator.Add else "xg_dsub_i"
                     return f"{fn}((double)({lc}), (double)({rc}))"
-                return f"({lc} {e.operator.value} {rc})"
+                if not fma64:
+                    return f"({lc} {e.operator.value} {rc})"
+            if fma64 and e.operator in FMA64 and self.ctype(e) == "double":
+                return f"{FMA64[e.operator]}({self.fma64_operand(e.left, env)}, {self.fma64_operand(e.right, env)}, xg_f)"
             return f"({self.expr(e.left, env)} {e.operator.value} {self.expr(e.right, env)})"
         if isinstance(e, ir.Call):
             return self.call(e, env)
         raise TypeError(f"cannot emit {type(e).__name__}")
+
+    def fma64_operand(self, e: ir.Expression, env) -> str:
+        """An operand of an FP64 operation in a vector register (launch constants
+        would otherwise be read from the constant bank, at the slower rate)."""
+        code = f"(double)({self.expr(e, env)})"
+        return f"xg_vreg({code}, xg_f)" if isinstance(e, ir.Constant) or env.substitute(e) is not None else code
 
     def call(self, e: ir.Call, env) -> str:
         from .operator import Operator
@@ -893,6 +909,7 @@ class SweepEnv:
         self.div_map = div_map or {}
         self.mul_map = mul_map or {}
         self.int_adds = int(getattr(gen.cfg, "int_adds", 0))
+        self.fma64 = bool(gen.cfg.exact)  # exact=False lets the compiler contract plain operators instead
         self.add_count = 0
         self.add_memo: dict = {}
 
@@ -975,6 +992,8 @@ def zstage_frame(kname: str, ptype: str, T: str, srcs: list, loads: list, outs: 
          "  extern __shared__ __align__(16) unsigned char xg_zs_raw[];",
          f"  {T}* const ring = ({T}*)xg_zs_raw;  // [R][NB][PY][PX]",
          "  const int tid = threadIdx.x;",
+         "  const xg_fp64 xg_f = xg_fp64_units();",
+         "  (void)xg_f;",
          "  const int ntx = (int)((p.X + TX - 1) / TX), nty = (int)((p.Y + TY - 1) / TY);",
          "  const int ix = blockIdx.x % ntx, iy = (blockIdx.x / ntx) % nty, iz = blockIdx.x / (ntx * nty);",
          "  const int x0 = ix * TX, y0 = iy * TY, z0 = iz * zlen;",
@@ -1918,7 +1937,8 @@ class SweepGroupEmitter:
         dst = self.bname((s.slot, s.level, s.write_version))
         pre, val = self.value_code(s, False, "    ")
         K = [f"__global__ void __launch_bounds__(256) xgk_{n}_{gid}_{tag}(const __grid_constant__ "
-             f"struct xgp_{n}_{gid}_{tag} p) {{"] + self.restrict_locals(sweeps) + [
+             f"struct xgp_{n}_{gid}_{tag} p) {{", "  const xg_fp64 xg_f = xg_fp64_units();",
+             "  (void)xg_f;"] + self.restrict_locals(sweeps) + [
              "  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < p.ncells; "
              "e += (int64_t)gridDim.x * blockDim.x) {",
              "    const int64_t c = p.cells[e];",

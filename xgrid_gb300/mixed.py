@@ -252,7 +252,7 @@ class MixedLoopEmitter:
                      extra_args=", float* mx_r, float* mx_d, int64_t mx_pad, float* mx_max",
                      extra_fill=["  p.mx_r = mx_r; p.mx_d = mx_d; p.mx_pad = mx_pad; p.mx_max = mx_max;"],
                      final=(["float xg_amax = 0.f;"],
-                            [f"const float rr = (float)({S}[c] - {P0}[c]);",
+                            [f"const float rr = (float)xg_dsub({S}[c], {P0}[c], xg_f);",
                              "const I xa = c + ((I)z * (I)p.Y + (I)y) * (I)p.mx_pad;",
                              "p.mx_r[xa] = rr;",
                              "if (p.mx_d) p.mx_d[xa] = rr;",
@@ -399,7 +399,7 @@ class MixedLoopEmitter:
              "      const float dv = p.mx_kind == 0 ? ((const float*)p.mx_d)[xa] : (p.mx_kind == 1 ? "
              "__half2float(((const __half*)p.mx_d)[xa]) : __bfloat162float(((const __nv_bfloat16*)p.mx_d)[xa])) "
              "* xg_inv;",
-             f"      {P}[c] = {P}[c] + (double)dv;", "    }}"]
+             f"      {P}[c] = xg_dadd({P}[c], (double)dv, xg_f);", "    }}"]
         for j in bnds:
             s = sweeps[j]
             pre, val = b.value_code(s, False, "    ")

@@ -37,8 +37,8 @@ from __future__ import annotations
 from . import analysis
 
 THREADS = 256
-SITE = 57
-MIN_BLOCKS = 2  # resident CTAs per SM asked of ptxas  # profiling site of the launch within its group
+SITE = 57  # profiling site of the launch within its group
+MIN_BLOCKS = 4  # resident CTAs per SM asked of ptxas (the boxes of a wave are sized for four)
 
 
 def plan(em) -> dict | None:
@@ -139,6 +139,8 @@ def emit(em, th: int) -> None:
          "  const int Y = (int)p.Y, X = (int)p.X;",
          "  const bool zero = p.bzero[b] != 0;",
          "  const int tid = threadIdx.x;",
+         "  const xg_fp64 xg_f = xg_fp64_units();",
+         "  (void)xg_f;",
          f"  const {T}* __restrict__ tin = p.{src};",
          "  // the box of the target (and of the mask when it holds boundary cells); beyond the grid: 0",
          "  for (int l = tid; l < NB; l += NT) {",
