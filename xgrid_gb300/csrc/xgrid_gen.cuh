@@ -91,7 +91,10 @@ __device__ __forceinline__ double xg_dsq(double a, const xg_fp64& f) { return __
 //     q  = RN(x*zh + RN(x*zl))        within 1 ulp of x/d (a faithful quotient)
 //     r  = x - q*d                    exact (one fma) for a faithful q
 //     q' = RN(q + r*zh)               = RN(x/d) by Markstein's theorem
-// as long as nothing underflows or overflows.  The host derives from d the
+// as long as nothing underflows or overflows.  For most divisors q itself is
+// already RN(x/d) for every x, which the host proves per divisor
+// (xg_two_op_divisor): two FP64 operations instead of four (cavity step at 1500^2,
+// where no divisor is a power of two: 3339 -> 2594 us).  The host derives from d the
 // window of x exponents where that holds; outside it (and for d not normal,
 // x = 0, inf, NaN, tiny or huge) the IEEE division runs instead, so the result
 // is RN(x/d) for every x.
@@ -139,8 +142,49 @@ struct xg_divisor {
   double d, zh, zl;
   unsigned lo, span;  // fast path when (biased exponent of x) - lo <= span (unsigned)
   int ok;
+  int two;            // RN(x*zh + RN(x*zl)) is RN(x/d) for every x of the window
   xg_scale rz;        // d = +-2^s: x/d = x * 2^-s exactly (rz.p2 set)
 };
+
+// Whether v = RN(x*zh + u), u = RN(x*zl), is RN(x/d) for every double x with
+// normal intermediates: the two-operation product by a constant of Brisebarre &
+// Muller, "Correctly rounded multiplication by arbitrary precision constants",
+// IEEE Trans. Computers 57(2), 2008, with the hard cases enumerated.  Before its
+// rounding v is within 2^-52 |x zl| <= 2^-105 |x/d| of x/d (half an ulp of zl and of
+// u each), so v can only be wrong where x/d lies that close to a midpoint m of two
+// doubles.  With integer significands X of x, D of |d| in [2^52, 2^53) and an odd M
+// in (2^53, 2^54), m = M 2^-53 when X >= D (quotient in [1, 2)) and M 2^-54 when
+// X < D, and the distance is |X 2^k - M D| / (D 2^k) with k = 53 or 54: the integer
+// R = X 2^k - M D has |R| <= 2 or |R| <= 4.  Each R fixes M modulo 2^k / gcd, so a
+// handful of x remain, and each is tried.  (R = 0 would need 2^k to divide D.)
+static inline bool xg_two_op_divisor(double d) {
+  int ex = 0;
+  const double dn = ldexp(frexp(fabs(d), &ex), 53);  // the significand: an integer in [2^52, 2^53)
+  const uint64_t D = (uint64_t)dn;
+  const double zh = 1.0 / dn, zl = fma(-zh, dn, 1.0) / dn;
+  int t = 0;
+  while (!((D >> t) & 1)) ++t;
+  const uint64_t Do = D >> t;
+  uint64_t inv = Do;  // inverse of the odd part modulo 2^64 (Newton: five doublings from 3 bits)
+  for (int i = 0; i < 5; ++i) inv *= 2 - Do * inv;
+  for (int k = 53; k <= 54; ++k) {
+    const int rmax = k == 53 ? 2 : 4;
+    for (int r = -rmax; r <= rmax; ++r) {
+      if (r == 0 || (r & ((1 << (t < 4 ? t : 4)) - 1)) != 0 || t > 2) continue;  // 2^t divides R
+      const uint64_t mod = (uint64_t)1 << (k - t);
+      const uint64_t m0 = ((uint64_t)(-(int64_t)r >> t) * inv) & (mod - 1);  // M Do = -R / 2^t (mod 2^(k-t))
+      for (uint64_t M = m0; M < ((uint64_t)1 << 54); M += mod) {
+        if (M <= ((uint64_t)1 << 53) || !(M & 1)) continue;
+        const unsigned __int128 XK = (unsigned __int128)M * D + (unsigned __int128)(__int128)r;
+        const uint64_t X = (uint64_t)(XK >> k);
+        if ((unsigned __int128)X << k != XK || X < ((uint64_t)1 << 52) || X >= ((uint64_t)1 << 53)) continue;
+        const double x = (double)X;
+        if (fma(x, zh, x * zl) != x / dn) return false;
+      }
+    }
+  }
+  return true;
+}
 
 static inline xg_divisor xg_make_divisor(double d) {
   xg_divisor k;
@@ -163,6 +207,7 @@ static inline xg_divisor xg_make_divisor(double d) {
   k.lo = (unsigned)(lo + 1023);
   k.span = (unsigned)(hi - lo);
   k.ok = 1;
+  k.two = (k.zl == 0.0 || fpclassify(k.zl) == FP_NORMAL) && xg_two_op_divisor(d) ? 1 : 0;
   return k;
 }
 
@@ -173,6 +218,7 @@ __device__ __forceinline__ double xg_divk(double x, const xg_divisor& k, const x
   if (k.ok && e - k.lo <= k.span) {
     const double zh = xg_vreg(k.zh, f);
     const double q = __fma_rn(x, zh, xg_dmul(x, xg_vreg(k.zl, f), f));
+    if (k.two) return q;
     const double r = __fma_rn(-q, xg_vreg(k.d, f), x);
     return __fma_rn(r, zh, q);
   }
