@@ -370,7 +370,7 @@ class BatchEmitter:
         from .codegen import HostEnv
         H += e.host_hoists(HostEnv(gen), "      ")[2:]
         H += ["    }", "    const struct xgh_" + n + "_" + str(gid) + "* h = &xg_h;"]
-        H += ["    " + l.strip() for l in e.fill_params("batch", g.sweeps, g.sweeps[0].slot)]
+        H += ["    " + l.strip() for l in e.fill_params("batch", g.sweeps, g.sweeps[0].slot, auto=False)]
         H += [f"    if (!p.same) XG_FAIL(\"{n}: every grid of a batched problem needs the same shape\");",
               "    int64_t ntiles = 0;"]
         for j in mains:

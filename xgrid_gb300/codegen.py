@@ -47,6 +47,12 @@ OVERSTEP = {"none": "XG_OVERSTEP_NONE", "limit": "XG_OVERSTEP_LIMIT", "wrap": "X
 ZWALK_PLANES = 4
 ZWALK_BLOCKS = 4
 
+# FP64 launches: rows per thread and iteration of one main sweep, resident CTAs per SM asked of
+# ptxas (4097^2 Jacobi sweep: 4 rows and 4 CTAs 189 us, 2 and 4 165, 2 and 5 154, 2 and 6 151,
+# where 512^2 heat takes 7.1, 7.5 and 7.6 with 4, 5 and 6 CTAs), and the operations per cell from
+# which two CTAs are enough (min_blocks)
+ROWS_WIDE, BLOCKS_WIDE, FP64_HEAVY = 2, 5, 40
+
 # staged z-walk of mask-free 3-D sweeps: (y, x) column block of a CTA, thread rows, planes
 # prefetched beyond the next one (chunk lengths along z: xg_zstage_chunks)
 ZSTAGE_TILE = (8, 128)
@@ -579,6 +585,7 @@ class CudaGenerator:
         for gi in range(max(self.group_counter[0], 1)):
             src.append("  {" + ", ".join(str(v) for v in self.group_tiling.get(gi, DEFAULT_TILING[2])) + "},")
         src.append("};")
+        src.append(f"static uint8_t xg_tiling_set_{name}[{max(self.group_counter[0], 1)}];  // set by xg_config: used as is")
         batch_host = None
         from . import batch as batch_mod
         if (not device_only and batch_mod.qualifies(self) and len(self.group_emitters) == 1
@@ -595,6 +602,7 @@ class CudaGenerator:
         src.append(f"  if (fuse >= 0) xg_fuse_{name} = fuse;")
         src.append(f"  if (group < 0 || group >= {self.group_counter[0]} || !cfg) return 0;")
         src.append(f"  for (int i = 0; i < 6; ++i) xg_tiling_{name}[group][i] = cfg[i];")
+        src.append(f"  xg_tiling_set_{name}[group] = 1;")
         src.append("  return 0;")
         src.append("}")
         src.append(f'extern "C" int xg_groups_{name}(void) {{ return {self.group_counter[0]}; }}')
@@ -1355,12 +1363,23 @@ class SweepGroupEmitter:
                 out.append(b[0])
         return out
 
+    def wide(self) -> bool:
+        """Whether the group sweeps FP64 grids."""
+        return any(self.elem(b[0]) == "double" for b in self.buffers(self.g.sweeps))
+
     def min_blocks(self) -> int:
-        """Resident 256-thread CTAs per SM asked of ptxas: FP64 sweeps are bound by
-        the FP64 pipe and keep registers for ILP; FP32/integer sweeps are memory
-        bound and want occupancy."""
-        wide = any(self.elem(b[0]) == "double" for b in self.buffers(self.g.sweeps))
-        return 4 if wide else 6
+        """Resident 256-thread CTAs per SM asked of ptxas.  FP32 and integer sweeps
+        are memory bound and want occupancy; so do FP64 sweeps of few operations
+        (4097^2 source group of 25: 543 us with 4 or 5 CTAs, 596 with 2).  Launches of
+        many FP64 operations a cell are bound by the FP64 pipe, which a few warps
+        fill when the registers let loads run ahead (momentum group of 48: 1145 us
+        with 2 CTAs, 1290 with 4)."""
+        if not self.wide():
+            return 6
+        ops = sum(isinstance(e, ir.Binary) and not e.operator.is_compare() and not e.operator.is_logic()
+                  and has_stencil(e) and self.gen.ctype(e) == "double"
+                  for s in self.g.sweeps if s.is_main for e in ir.walk(s.stmt.value))
+        return 2 if ops >= FP64_HEAVY else BLOCKS_WIDE
 
     def restrict_locals(self, sweeps) -> list:
         """Kernel-local __restrict__ copies of the buffer pointers: distinct buffer
@@ -1626,7 +1645,7 @@ class SweepGroupEmitter:
         if not all(self.elem(b[0]) in numeric for b in self.buffers([s])):
             return 0
         nl = len(s.distinct_loads()) + (1 if s.implicit else 0)
-        return 4 if nl <= 6 else (2 if nl <= 12 else 0)
+        return (ROWS_WIDE if self.wide() else 4) if nl <= 6 else (2 if nl <= 12 else 0)
 
     def rows_loop(self, j: int, mask_var: str, indent: str = "  ", mode: str = "fast", R: int = 4) -> list:
         """Cell loop that walks ``R`` rows per thread and iteration in two phases:
@@ -1808,12 +1827,23 @@ class SweepGroupEmitter:
         lines.append("}")
         return "\n".join(lines)
 
-    def fill_params(self, tag: str, sweeps, dom_slot: int, single=None, indent: str = "  ") -> list:
+    def tiling_lines(self, slot, indent: str = "  ") -> list:
+        """``tl``: this group's tiling for the grid in ``slot`` (None: as configured)."""
+        n, gid = self.name, self.gid
+        if slot is None:
+            return [f"{indent}const int32_t* tl = xg_tiling_{n}[{gid}];"]
+        return [f"{indent}int32_t tl_[6];",
+                f"{indent}const int32_t* tl = xg_tiling_for(xg_tiling_{n}[{gid}], xg_tiling_set_{n}[{gid}], "
+                f"&G[{slot}], tl_);",
+                f"{indent}if (!tl) return -1;"]
+
+    def fill_params(self, tag: str, sweeps, dom_slot: int, single=None, indent: str = "  ",
+                    auto: bool = True) -> list:
         n, gid = self.name, self.gid
         lines = [f"{indent}struct xgp_{n}_{gid}_{tag} p;",
                  f"{indent}memset(&p, 0, sizeof p);",
                  f"{indent}p.h = *h;",
-                 f"{indent}const int32_t* tl = xg_tiling_{n}[{gid}];",
+                 *self.tiling_lines(dom_slot if auto else None, indent),
                  f"{indent}xg_ext dom = xg_extent(&G[{dom_slot}]);",
                  f"{indent}p.Z = dom.z; p.Y = dom.y; p.X = dom.x;",
                  f"{indent}p.tz = tl[0]; p.ty = tl[1]; p.tx = tl[2];",

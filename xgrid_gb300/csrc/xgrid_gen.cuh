@@ -332,6 +332,49 @@ static inline int64_t xg_tiles_along(int64_t n, int32_t t) {
   return t < 0 ? (n < -(int64_t)t ? n : -(int64_t)t) : (n / t > 0 ? n / t : 1);
 }
 
+// The device's SM count (asked once).
+static inline int xg_sm_count(int* sms) {
+  static int n = 0;
+  if (n == 0) {
+    int dev = 0, v = 0;
+    XG_CUDA(cudaGetDevice(&dev));
+    XG_CUDA(cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev));
+    n = v > 0 ? v : 1;
+  }
+  *sms = n;
+  return 0;
+}
+
+// The tiling of a launch: `cfg` when it was set for the group, else on 2-D grids the
+// default's columns and threads, and a tile count along y (a negative extent) that
+// spreads the cells evenly over the SMs where the default's rows do not.  A sweep that
+// is bound by an SM's FP64 pipe ends with the SM that holds the most tiles: the cost is
+// ceil(tiles / SMs) * (rows per tile + 2), two rows standing for a tile's own tables,
+// barriers and first loads.  The default stays when it costs at most a tenth more (the
+// loops take its 64 rows in whole passes, which a memory-bound sweep feels: 229 against
+// 250 us for the 4097^2 residual launch with 216 rows).  Tiles keep at least 4 rows, so
+// that boundary phases that read the row next to theirs stay inside the tile.
+static inline const int32_t* xg_tiling_for(const int32_t* cfg, int set, const xg_grid* g, int32_t* buf) {
+  if (set || g->ndim != 2) return cfg;
+  int sms = 0;
+  if (xg_sm_count(&sms) != 0) return NULL;
+  const xg_ext e = xg_extent(g);
+  const int64_t ntx = xg_tiles_along(e.x, cfg[2]), n0 = xg_tiles_along(e.y, cfg[1]);
+  int64_t best = -1, first = -1, count = n0;
+  for (int64_t n = n0; n == n0 || (n <= e.y / 4 && n <= n0 + 256); ++n) {
+    const int64_t cost = ((n * ntx + sms - 1) / sms) * ((e.y + n - 1) / n + 2);
+    if (first < 0) first = cost;
+    if (best < 0 || cost < best) {
+      best = cost;
+      count = n;
+    }
+  }
+  if (10 * first <= 11 * best || count > 65535) return cfg;
+  memcpy(buf, cfg, 6 * sizeof(int32_t));
+  buf[1] = -(int32_t)count;
+  return buf;
+}
+
 // The tile of the calling CTA: the launch grid is (ntx, nty, ntz) tiles, so the
 // tile coordinates are the block indices (no division); t is the linear tile id
 // used by the mask tables.
@@ -673,13 +716,8 @@ static inline int xg_smem_optin(K* kernel, int* avail) {
 // planes at half weight (neighbouring chunks read them too, often from L2).
 // Chunks hold at least 8 planes.  *nt receives the CTA count.
 static inline int xg_zstage_chunks(int64_t Z, int64_t Y, int64_t X, int ty, int tx, int* zlen, int64_t* nt) {
-  static int nsm = 0;
-  if (nsm == 0) {
-    int dev = 0;
-    XG_CUDA(cudaGetDevice(&dev));
-    XG_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    if (nsm < 1) nsm = 1;
-  }
+  int nsm = 0;
+  XG_TRY(xg_sm_count(&nsm));
   const int64_t ncb = ((X + tx - 1) / tx) * ((Y + ty - 1) / ty);
   int64_t cmax = Z / 8 > 1 ? Z / 8 : 1;
   if (cmax > 4096) cmax = 4096;

@@ -426,7 +426,7 @@ class MixedLoopEmitter:
               f"  if (!xg_fuse_{n} || !G[{slot}].scratch || !G[{slot}].aux) return 0;",
               "  xg_mx_aux A;",
               f"  if (xg_mx_layout(&G[{slot}], &A) != 0) return 0;",
-              f"  const int32_t* tl = xg_tiling_{n}[{gid}];"]
+              *b.tiling_lines(slot)]
         for j, offs in plan.group.local_checks:
             flat = ", ".join(str(v) for o in offs for v in o)
             L += ["  {", f"    static const int32_t offs[] = {{{flat}}};", "    int ok = 0;",
@@ -440,7 +440,7 @@ class MixedLoopEmitter:
               f"  struct xgp_{n}_{gid}_mxd p;",
               "  memset(&p, 0, sizeof p);",
               "  p.k = *hm;",
-              f"  const int32_t* tl = xg_tiling_{n}[{gid}];",
+              *b.tiling_lines(slot),
               f"  xg_ext e = xg_extent(&G[{slot}]);",
               "  p.Z = e.z; p.Y = e.y; p.X = e.x;",
               "  p.tz = tl[0]; p.ty = tl[1]; p.tx = tl[2];",
