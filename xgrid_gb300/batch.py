@@ -27,6 +27,8 @@ from __future__ import annotations
 from . import analysis, ir
 
 DEPTH_MAX = 8
+# resident CTAs per SM asked of ptxas for the register-block kernel of one and of two fields
+REG_BLOCKS = (3, 2)
 
 
 def qualifies(gen) -> bool:
@@ -80,6 +82,186 @@ class BatchEmitter:
             if t.dimension > 2:
                 return None
         return ry, rx
+
+    def reg_plan(self) -> bool:
+        """Whether the temporal steps can run on register blocks (``emit_reg``): FP32
+        fields on 2-D grids, every load within one cell on each axis."""
+        gen, g = self.gen, self.g
+        r = self.tb_plan()
+        if r is None or max(r) > 1:
+            return False
+        for s in g.sweeps:
+            t = gen.defn.signature.arguments[self.e.arg_index(s.slot)][1]
+            if self.e.elem(s.slot) != "float" or t.dimension != 2:
+                return False
+        return len(g.sweeps) <= 2
+
+    def emit_reg(self) -> str:
+        """Temporally blocked kernel on register blocks, ``xgk_<n>_tbr``.
+
+        Same work items, buffers and arithmetic per cell as ``xgk_<n>_tb``, whose
+        steps are bound by instruction issue (five shared loads, a store and their
+        addresses around nine FP32 operations: 41 instructions per cell).  Here a
+        box is 64 rows of 32 * C columns; a lane holds C columns of its warp's 8
+        rows in registers for all T steps.  A neighbour column comes from the next
+        lane (one shuffle per row and side), a row beyond the warp's block through
+        a double-buffered shared array (one barrier per step).  Every cell of the
+        box is computed in every step: what is stale at its rim moves inwards one
+        cell per step and the halo of T cells keeps it out of the tile.  Each warp
+        stages and stores its own rows through shared memory, so that global
+        accesses are contiguous over the lanes whatever the row's alignment."""
+        from .codegen import SweepEnv
+        gen, g, e = self.gen, self.g, self.e
+        n, gid = gen.op.name, g.index
+        ry, rx = self.tb_plan()
+        fields = [s.slot for s in g.sweeps]
+        offs = {f: set() for f in fields}
+        for s in g.sweeps:
+            for _, ld in s.loads:
+                offs[ld.slot].add((ld.offset[1], ld.offset[2]))
+        # rows whose neighbour columns are read: of the row itself only, or of the rows next to it too
+        side = {f: {oy for oy, ox in offs[f] if ox} for f in fields}
+        diag = {f: bool(side[f] - {0}) for f in fields}
+        row = {-1: "pv", 0: "cr", 1: "nx"}
+        K = [f"template <typename I, int C> __global__ void __launch_bounds__(256, {REG_BLOCKS[len(fields) - 1]}) "
+             f"xgk_{n}_tbr(const struct xgb_{n}* __restrict__ desc, const int64_t* __restrict__ tile0, int nprob, "
+             f"int64_t total, int T, int tby, int tbx, int in_idx, int out_idx, int prev_idx, "
+             f"unsigned long long* __restrict__ counter) {{",
+             f"  constexpr int NW = 8, RS = 8, BX = 32 * C, F = {len(fields)};",
+             "  constexpr unsigned FULL = 0xffffffffu;",
+             "  extern __shared__ __align__(16) unsigned char xg_smem[];  // [F][NW * RS][BX]",
+             "  __shared__ __align__(16) float ex[2][F][2][NW][BX];  // [parity][field][first/last row][warp][column]",
+             "  __shared__ int64_t item_;",
+             "  __shared__ int prob_;",
+             "  const xg_fp64 xg_f = xg_fp64_units();",
+             "  (void)xg_f;",
+             "  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, r0 = w * RS;",
+             "  float* const st = (float*)xg_smem;",
+             f"  const int HY = T * {ry}, HX = T * {rx};",
+             "  int64_t next = 0;",
+             "  if (tid == 0) next = (int64_t)atomicAdd(counter, 1ull);",
+             "  for (;;) {",
+             "    if (tid == 0) {",
+             "      const int64_t it = next;",
+             "      if (it < total) next = (int64_t)atomicAdd(counter, 1ull);",
+             "      int lo = 0, hi = nprob - 1;",
+             "      if (it < total)",
+             "        while (lo < hi) {",
+             "          const int mid = (lo + hi + 1) >> 1;",
+             "          if (tile0[mid] <= it) lo = mid; else hi = mid - 1;",
+             "        }",
+             "      item_ = it;",
+             "      prob_ = lo;",
+             "    }",
+             "    __syncthreads();",
+             "    const int64_t it = item_;",
+             "    const int pr = prob_;",
+             "    __syncthreads();",
+             "    if (it >= total) break;",
+             f"    const struct xgb_{n}& D = desc[pr];",
+             f"    const struct xgp_{n}_{gid}_batch& p = D.par;",
+             "    const int t = (int)(it - D.tile0tb);",
+             "    const int ntx = D.tbn[1];",
+             "    const int itx = t % ntx, ity = t / ntx;",
+             "    const int X = (int)p.X, Y = (int)p.Y;",
+             "    const int x0 = itx * tbx, y0 = ity * tby;",
+             "    const int RY = min(tby, Y - y0) + 2 * HY, RX = min(tbx, X - x0) + 2 * HX;",
+             "    const bool active = r0 < RY;  // the same for the whole warp",
+             "    // the warp's rows of the box, wrapped, lanes along the row",
+             "    if (active) {",
+             "      int gx[C];",
+             "#pragma unroll",
+             "      for (int c = 0; c < C; ++c) {",
+             "        const int x = x0 - HX + lane + 32 * c;",
+             "        gx[c] = x < 0 ? x + X : (x >= X ? x - X : x);",
+             "      }",
+             "#pragma unroll",
+             "      for (int i = 0; i < RS; ++i)",
+             "        if (r0 + i < RY) {",
+             "          int gy = y0 - HY + r0 + i;",
+             "          gy = gy < 0 ? gy + Y : (gy >= Y ? gy - Y : gy);",
+             "          const I gr = (I)gy * (I)X;",
+             "#pragma unroll",
+             "          for (int c = 0; c < C; ++c)",
+             "            if (lane + 32 * c < RX) {"]
+        for k, f in enumerate(fields):
+            K.append(f"              xg_cp_async(&st[({k} * NW * RS + r0 + i) * BX + lane + 32 * c], "
+                     f"(const float*)D.tb[{f}][in_idx] + gr + gx[c]);")
+        K += ["            }",
+              "        }",
+              "    }",
+              "    xg_cp_async_wait_all();",
+              "    __syncwarp();",
+              "    // the lane's block: columns C * lane .. of the warp's rows"]
+        for k, f in enumerate(fields):
+            K += [f"    float d{f}[RS][C];",
+                  "#pragma unroll",
+                  "    for (int i = 0; i < RS; ++i)",
+                  f"      xg_ldv<C>(d{f}[i], &st[({k} * NW * RS + r0 + i) * BX + C * lane]);"]
+        K += ["    // the tile's own cells of the warp's rows to level `lv` of the ring",
+              "    auto put = [&](int lv) {",
+              "      if (!active) return;",
+              "      __syncwarp();",
+              "#pragma unroll",
+              "      for (int i = 0; i < RS; ++i) {"]
+        K += [f"        xg_stv<C>(&st[({k} * NW * RS + r0 + i) * BX + C * lane], d{f}[i]);" for k, f in enumerate(fields)]
+        K += ["      }",
+              "      __syncwarp();",
+              "#pragma unroll",
+              "      for (int i = 0; i < RS; ++i) {",
+              "        const int ly = r0 + i;",
+              "        if (ly >= HY && ly < RY - HY) {",
+              "          const I gr = (I)(y0 + ly - HY) * (I)X + (I)(x0 - HX + lane);",
+              "#pragma unroll",
+              "          for (int c = 0; c < C; ++c)",
+              "            if (lane + 32 * c >= HX && lane + 32 * c < RX - HX) {"]
+        for k, f in enumerate(fields):
+            K.append(f"              ((float*)D.tb[{f}][lv])[gr + 32 * c] = st[({k} * NW * RS + ly) * BX + lane + 32 * c];")
+        K += ["            }",
+              "        }",
+              "      }",
+              "    };",
+              "    for (int s = 1; s <= T; ++s) {",
+              "      if (s == T && prev_idx >= 0) put(prev_idx);  // the values of step T - 1",
+              "      if (active) {"]
+        for k, f in enumerate(fields):
+            K += [f"        xg_stv<C>(&ex[s & 1][{k}][0][w][C * lane], d{f}[0]);",
+                  f"        xg_stv<C>(&ex[s & 1][{k}][1][w][C * lane], d{f}[RS - 1]);"]
+        K += ["      }", "      __syncthreads();", "      if (active) {",
+              "        // rows i - 1, i, i + 1 with the columns next to the block at [0] and [C + 1]"]
+        for k, f in enumerate(fields):
+            K += [f"        float pv{f}[C + 2], cr{f}[C + 2], nx{f}[C + 2], dn{f}[C];",
+                  f"        xg_ldv<C>(&pv{f}[1], &ex[s & 1][{k}][1][w > 0 ? w - 1 : 0][C * lane]);",
+                  f"        xg_ldv<C>(dn{f}, &ex[s & 1][{k}][0][w < NW - 1 ? w + 1 : w][C * lane]);",
+                  "#pragma unroll",
+                  f"        for (int j = 0; j < C; ++j) cr{f}[j + 1] = d{f}[0][j];"]
+            if diag[f]:
+                K.append(f"        xg_sides<C>(pv{f});")
+            if side[f]:
+                K.append(f"        xg_sides<C>(cr{f});")
+        K += ["#pragma unroll", "        for (int i = 0; i < RS; ++i) {"]
+        for f in fields:
+            K += ["#pragma unroll",
+                  f"          for (int j = 0; j < C; ++j) nx{f}[j + 1] = i + 1 < RS ? d{f}[i + 1 < RS ? i + 1 : i][j] : dn{f}[j];"]
+            if side[f]:
+                K.append(f"          {'' if diag[f] else 'if (i + 1 < RS) '}xg_sides<C>(nx{f});")
+        K += ["#pragma unroll", "          for (int j = 0; j < C; ++j) {"]
+        stores = []
+        for s in g.sweeps:
+            names, local = {}, {}
+            for st_, ld in s.loads:
+                if ld not in local:
+                    local[ld] = f"l{len(local)}_{s.slot}"
+                    K.append(f"            const float {local[ld]} = {row[ld.offset[1]]}{ld.slot}[j + 1 + ({ld.offset[2]})];")
+                names[id(st_)] = local[ld]
+            env = SweepEnv(gen, e.hoist_map, names, e.div_map, e.mul_map)
+            stores.append(f"            d{s.slot}[i][j] = {gen.expr(s.stmt.value, env)};")
+        K += stores + ["          }"]
+        for f in fields:
+            K += ["#pragma unroll",
+                  f"          for (int j = 0; j < C + 2; ++j) {{ pv{f}[j] = cr{f}[j]; cr{f}[j] = nx{f}[j]; }}"]
+        K += ["        }", "      }", "    }", "    put(out_idx);", "  }", "}"]
+        return "\n".join(K)
 
     def emit_tb(self) -> tuple:
         """Temporally blocked persistent kernel ``xgk_<n>_tb`` and its host entry
@@ -193,7 +375,28 @@ class BatchEmitter:
         K += [f"          if (prev_idx >= 0) prv{f}[row + lx] = c{f}[c];" for f in fields]
         K += ["        }", "      }", "    }", "  }", "}"]
 
+        reg = self.reg_plan()
+        if reg:
+            K.append(self.emit_reg())
         smem = " + ".join(f"(((size_t)PX * PY * sizeof({el[f]}) + 15) & ~(size_t)15) * 2" for f in fields)
+        reg_blocks, reg_launch = [], []
+        if reg:
+            reg_blocks = [f"  if (const int C = xg_tb_reg_{n}(T, ty, tx)) {{",
+                          f"    const size_t bytes = (size_t)64 * 32 * C * sizeof(float) * {len(fields)};"]
+            for c in (2, 4):
+                for it in ("int", "int64_t"):
+                    reg_blocks.append(f"    if (C == {c}) XG_TRY(xg_smem_optin(xgk_{n}_tbr<{it}, {c}>, &cap));")
+                reg_blocks.append(f"    if (C == {c}) XG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, "
+                                  f"xgk_{n}_tbr<int, {c}>, 256, bytes));")
+            reg_blocks += ["    if (per < 1) XG_FAIL(\"temporal blocking: no CTA of the register-block kernel fits an "
+                           "SM\");",
+                           "    *smem = (int)bytes;", "    *blocks = sms * per;", "    return 0;", "  }"]
+            for c in (2, 4):
+                for it, cond in (("int", "b.small"), ("int64_t", "!b.small")):
+                    reg_launch.append(f"    {'else ' if reg_launch else ''}if (C == {c} && {cond}) "
+                                      f"xgk_{n}_tbr<{it}, {c}><<<b.blocks, 256, b.smem, s>>>(d, t0, b.nprob, b.total, "
+                                      "dep, b.ty, b.tx, in, out, prev, b.counters + i);")
+            reg_launch.append("    else")
         H = [f"struct xgbt_{n} {{ const void* desc; int64_t total; int64_t steps; unsigned long long* counters; "
              f"int32_t nprob; int32_t small; int32_t blocks; int32_t T; int32_t ty; int32_t tx; int32_t smem; "
              f"int32_t block[3]; }};",
@@ -201,13 +404,20 @@ class BatchEmitter:
              f"  const size_t PX = (size_t)tx + 2 * (size_t)T * {rx}, PY = (size_t)ty + 2 * (size_t)T * {ry};",
              f"  return {smem};",
              "}",
+             "// columns per lane (2 or 4) of the register-block kernel whose box of 64 rows and 64 or 128",
+             "// columns holds a tile and its halo, 0: none does and the shared-memory kernel runs",
+             f"static int xg_tb_reg_{n}(int T, int ty, int tx) {{",
+             f"  if (!{int(reg)} || ty + 2 * T * {ry} > 64 || tx + 2 * T * {rx} > 128) return 0;",
+             f"  return tx + 2 * T * {rx} > 64 ? 4 : 2;",
+             "}",
              f'extern "C" int xg_batch_tb_blocks_{n}(int block_threads, int T, int ty, int tx, int* smem, '
              f'int* blocks) {{',
              "  if (T < 1 || ty < 1 || tx < 1) XG_FAIL(\"temporal blocking: T, ty and tx must be positive\");",
-             f"  const size_t bytes = xg_tb_smem_{n}(T, ty, tx);",
              "  int dev = 0, sms = 0, per = 0, cap = 0, cap64 = 0;",
              "  XG_CUDA(cudaGetDevice(&dev));",
              "  XG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));",
+             *reg_blocks,
+             f"  const size_t bytes = xg_tb_smem_{n}(T, ty, tx);",
              f"  XG_TRY(xg_smem_optin(xgk_{n}_tb<int>, &cap));",
              f"  XG_TRY(xg_smem_optin(xgk_{n}_tb<int64_t>, &cap64));",
              "  if (cap64 < cap) cap = cap64;",
@@ -237,6 +447,8 @@ class BatchEmitter:
              "  dim3 block(b.block[0], b.block[1], b.block[2]);",
              f"  const struct xgb_{n}* d = (const struct xgb_{n}*)b.desc;",
              "  const int64_t* t0 = (const int64_t*)(d + b.nprob) + b.nprob;",
+             f"  const int C = xg_tb_reg_{n}(b.T, b.ty, b.tx);",
+             "  (void)C;",
              "  int in = 0;",
              "  for (int64_t i = 0; i < L; ++i) {",
              "    const int dep = (int)(b.steps / L + (i < b.steps % L ? 1 : 0));",
@@ -245,6 +457,7 @@ class BatchEmitter:
              "    else if (i == L - 2) out = 2;",
              "    else out = 1 - in;",
              f"    xg_prof_launch({gid * 64 + 58}, s);",
+             *reg_launch,
              f"    if (b.small) xgk_{n}_tb<int><<<b.blocks, block, b.smem, s>>>(d, t0, b.nprob, b.total, dep, b.ty, "
              "b.tx, in, out, prev, b.counters + i);",
              f"    else xgk_{n}_tb<int64_t><<<b.blocks, block, b.smem, s>>>(d, t0, b.nprob, b.total, dep, b.ty, "

@@ -821,3 +821,28 @@ template <int N>
 __device__ __forceinline__ void xg_cp_async_wait_group() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
+
+// ---------------------------------------------------------------------------
+// Register blocks: C consecutive FP32 columns per lane (C = 2 or 4).
+template <int C>
+__device__ __forceinline__ void xg_ldv(float* d, const float* src) {
+  if (C == 4) {
+    const float4 v = *reinterpret_cast<const float4*>(src);
+    d[0] = v.x, d[1] = v.y, d[C - 2] = v.z, d[C - 1] = v.w;
+  } else {
+    const float2 v = *reinterpret_cast<const float2*>(src);
+    d[0] = v.x, d[1] = v.y;
+  }
+}
+template <int C>
+__device__ __forceinline__ void xg_stv(float* dst, const float* d) {
+  if (C == 4) *reinterpret_cast<float4*>(dst) = make_float4(d[0], d[1], d[C - 2], d[C - 1]);
+  else *reinterpret_cast<float2*>(dst) = make_float2(d[0], d[1]);
+}
+// A row with its neighbour columns: r[1 .. C] is the lane's, r[0] and r[C + 1] come
+// from the lanes next to it (the first and last lane keep a value of their own).
+template <int C>
+__device__ __forceinline__ void xg_sides(float* r) {
+  r[0] = __shfl_up_sync(0xffffffffu, r[C], 1);
+  r[C + 1] = __shfl_down_sync(0xffffffffu, r[1], 1);
+}
