@@ -1,5 +1,5 @@
 """Register-block kernel of the batched path: tiles whose box (tile and halo) just fits
-its 64 rows and 64 or 128 columns, smaller and remainder tiles, one field and two with
+its 64 or 128 rows and columns, smaller and remainder tiles, one field and two with
 diagonal loads, every depth's ring of levels -- the bits of one call per problem per step."""
 import numpy as np
 import pytest
@@ -21,7 +21,7 @@ def rows2d(u: xgrid.grid[float, 2], a: float) -> None:
 
 
 @pytest.mark.parametrize("temporal,steps", [((6, 52, 116), 12), ((6, 52, 52), 13), ((2, 60, 124), 5), ((1, 30, 30), 3),
-                                             ((8, 48, 112), 31), ((3, 7, 59), 6), ((4, 56, 57), 9), ((5, 54, 1), 10)])
+                                             ((8, 48, 112), 31), ((12, 104, 104), 25), ((3, 7, 59), 6), ((4, 56, 57), 9), ((5, 54, 1), 10)])
 @pytest.mark.parametrize("program", ["convdiff2d", "coupled2d", "rows2d"])
 def test_register_blocks_equal_sequential_calls(cacheroot, program, temporal, steps):
     xgrid.init(precision="float", cacheroot=cacheroot, opt_level=3, overstep="wrap")

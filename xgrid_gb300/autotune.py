@@ -126,12 +126,13 @@ def batch_candidates(one_dim: bool) -> list:
             for tx in (512, 1024, 2048):
                 out.append((d, 1, tx - 2 * d, (256, 1, 1)))
         return out
-    # tiles whose halo fills a box of 64 rows and 64 or 128 columns (register blocks), and tiles
-    # of the shared-memory kernel that FP64 fields and wider stencils take
+    # tiles whose halo fills a box of 64 or 128 rows and columns (register blocks), and tiles of
+    # the shared-memory kernel that FP64 fields and wider stencils take
     out = [(1, 32, 64, (32, 8, 1))]
-    for d in (2, 3, 4, 6, 8):
-        for ty, tx in ((64 - 2 * d, 128), (64 - 2 * d, 64), (16, 64), (32, 64), (32, 128), (64, 128)):
-            out.append((d, ty, tx - 2 * d, (32, 8, 1)))
+    for d in (2, 4, 6, 8, 12):
+        h = 2 * d
+        out += [(d, ty - h, tx - h, (32, 8, 1)) for ty in (64, 128) for tx in (64, 128)]
+        out += [(d, 32, tx - h, (32, 8, 1)) for tx in (64, 128)]
     return out
 
 

@@ -27,8 +27,12 @@ from __future__ import annotations
 from . import analysis, ir
 
 DEPTH_MAX = 8
-# resident CTAs per SM asked of ptxas for the register-block kernel of one and of two fields
-REG_BLOCKS = (3, 2)
+# register-block kernel: rows per warp and resident CTAs (of 8 warps) per SM asked of ptxas, by
+# fields.  16 rows make boxes of 128 rows, less of them halo and fewer barriers per cell: 15.0 us
+# a step for 60 problems of 64 to 1024 cells a side against 16.7 with 8 rows and 64-row boxes,
+# which spread little work better (8 problems of 64 to 512: 1.5 us a step against 1.9 with 4 warps
+# of 16 rows).  (Two cells in one packed FP32 instruction: 17 to 19 us.)
+REG_ROWS = (((8, 3), (16, 2)), ((8, 2),))
 
 
 def qualifies(gen) -> bool:
@@ -102,8 +106,8 @@ class BatchEmitter:
         Same work items, buffers and arithmetic per cell as ``xgk_<n>_tb``, whose
         steps are bound by instruction issue (five shared loads, a store and their
         addresses around nine FP32 operations: 41 instructions per cell).  Here a
-        box is 64 rows of 32 * C columns; a lane holds C columns of its warp's 8
-        rows in registers for all T steps.  A neighbour column comes from the next
+        box is NW * RS rows of 32 * C columns; a lane holds C columns of its warp's
+        RS rows in registers for all T steps.  A neighbour column comes from the next
         lane (one shuffle per row and side), a row beyond the warp's block through
         a double-buffered shared array (one barrier per step).  Every cell of the
         box is computed in every step: what is stale at its rim moves inwards one
@@ -123,11 +127,13 @@ class BatchEmitter:
         side = {f: {oy for oy, ox in offs[f] if ox} for f in fields}
         diag = {f: bool(side[f] - {0}) for f in fields}
         row = {-1: "pv", 0: "cr", 1: "nx"}
-        K = [f"template <typename I, int C> __global__ void __launch_bounds__(256, {REG_BLOCKS[len(fields) - 1]}) "
+        blocks = REG_ROWS[len(fields) - 1]
+        bound = f"RS == 16 ? {blocks[-1][1]} : {blocks[0][1]}"
+        K = [f"template <typename I, int C, int RS> __global__ void __launch_bounds__(256, {bound}) "
              f"xgk_{n}_tbr(const struct xgb_{n}* __restrict__ desc, const int64_t* __restrict__ tile0, int nprob, "
              f"int64_t total, int T, int tby, int tbx, int in_idx, int out_idx, int prev_idx, "
              f"unsigned long long* __restrict__ counter) {{",
-             f"  constexpr int NW = 8, RS = 8, BX = 32 * C, F = {len(fields)};",
+             f"  constexpr int NW = 8, BX = 32 * C, F = {len(fields)};",
              "  constexpr unsigned FULL = 0xffffffffu;",
              "  extern __shared__ __align__(16) unsigned char xg_smem[];  // [F][NW * RS][BX]",
              "  __shared__ __align__(16) float ex[2][F][2][NW][BX];  // [parity][field][first/last row][warp][column]",
@@ -227,24 +233,30 @@ class BatchEmitter:
         for k, f in enumerate(fields):
             K += [f"        xg_stv<C>(&ex[s & 1][{k}][0][w][C * lane], d{f}[0]);",
                   f"        xg_stv<C>(&ex[s & 1][{k}][1][w][C * lane], d{f}[RS - 1]);"]
-        K += ["      }", "      __syncthreads();", "      if (active) {",
-              "        // rows i - 1, i, i + 1 with the columns next to the block at [0] and [C + 1]"]
-        for k, f in enumerate(fields):
-            K += [f"        float pv{f}[C + 2], cr{f}[C + 2], nx{f}[C + 2], dn{f}[C];",
-                  f"        xg_ldv<C>(&pv{f}[1], &ex[s & 1][{k}][1][w > 0 ? w - 1 : 0][C * lane]);",
-                  f"        xg_ldv<C>(dn{f}, &ex[s & 1][{k}][0][w < NW - 1 ? w + 1 : w][C * lane]);",
-                  "#pragma unroll",
-                  f"        for (int j = 0; j < C; ++j) cr{f}[j + 1] = d{f}[0][j];"]
-            if diag[f]:
-                K.append(f"        xg_sides<C>(pv{f});")
-            if side[f]:
-                K.append(f"        xg_sides<C>(cr{f});")
-        K += ["#pragma unroll", "        for (int i = 0; i < RS; ++i) {"]
+        K.append("      }")
+        # two columns a lane leave the row loop little to overlap a shuffle with: all of them first
+        # (8 problems of 64 to 512 cells a side: 1.5 us a step against 2.4); four columns take each
+        # row's when the row comes (60 problems: 15.0 us a step against 17.2)
+        K.append("      constexpr bool pre = C == 2;")
         for f in fields:
-            K += ["#pragma unroll",
-                  f"          for (int j = 0; j < C; ++j) nx{f}[j + 1] = i + 1 < RS ? d{f}[i + 1 < RS ? i + 1 : i][j] : dn{f}[j];"]
             if side[f]:
-                K.append(f"          {'' if diag[f] else 'if (i + 1 < RS) '}xg_sides<C>(nx{f});")
+                K += [f"      float w{f}[RS + 2], e{f}[RS + 2];  // columns next to the block, rows -1 .. RS",
+                      "#pragma unroll",
+                      "      for (int i = 0; i < RS; ++i)",
+                      f"        if (pre || i == 0) xg_sides<C>(d{f}[i], w{f}[i + 1], e{f}[i + 1]);"]
+        K += ["      __syncthreads();", "      if (active) {"]
+        for k, f in enumerate(fields):
+            K += [f"        float pv{f}[C], cr{f}[C], nx{f}[C], dn{f}[C];  // rows i - 1, i, i + 1; row RS",
+                  f"        xg_ldv<C>(pv{f}, &ex[s & 1][{k}][1][w > 0 ? w - 1 : 0][C * lane]);",
+                  f"        xg_ldv<C>(dn{f}, &ex[s & 1][{k}][0][w < NW - 1 ? w + 1 : w][C * lane]);"]
+            if diag[f]:
+                K += [f"        xg_sides<C>(pv{f}, w{f}[0], e{f}[0]);", f"        xg_sides<C>(dn{f}, w{f}[RS + 1], e{f}[RS + 1]);"]
+        K += ["#pragma unroll", "        for (int i = 0; i < RS; ++i) {",
+              "#pragma unroll", "          for (int j = 0; j < C; ++j) {"]
+        K += [f"            cr{f}[j] = d{f}[i][j];" for f in fields]
+        K += [f"            nx{f}[j] = i + 1 < RS ? d{f}[i + 1 < RS ? i + 1 : i][j] : dn{f}[j];" for f in fields]
+        K.append("          }")
+        K += [f"          if (!pre && i + 1 < RS) xg_sides<C>(nx{f}, w{f}[i + 2], e{f}[i + 2]);" for f in fields if side[f]]
         K += ["#pragma unroll", "          for (int j = 0; j < C; ++j) {"]
         stores = []
         for s in g.sweeps:
@@ -252,14 +264,16 @@ class BatchEmitter:
             for st_, ld in s.loads:
                 if ld not in local:
                     local[ld] = f"l{len(local)}_{s.slot}"
-                    K.append(f"            const float {local[ld]} = {row[ld.offset[1]]}{ld.slot}[j + 1 + ({ld.offset[2]})];")
+                    (_, oy, ox), f = ld.offset, ld.slot
+                    at = f"{row[oy]}{f}[j]" if ox == 0 else (
+                        f"j > 0 ? {row[oy]}{f}[j > 0 ? j - 1 : 0] : w{f}[i + {1 + oy}]" if ox < 0 else
+                        f"j < C - 1 ? {row[oy]}{f}[j < C - 1 ? j + 1 : j] : e{f}[i + {1 + oy}]")
+                    K.append(f"            const float {local[ld]} = {at};")
                 names[id(st_)] = local[ld]
             env = SweepEnv(gen, e.hoist_map, names, e.div_map, e.mul_map)
             stores.append(f"            d{s.slot}[i][j] = {gen.expr(s.stmt.value, env)};")
-        K += stores + ["          }"]
-        for f in fields:
-            K += ["#pragma unroll",
-                  f"          for (int j = 0; j < C + 2; ++j) {{ pv{f}[j] = cr{f}[j]; cr{f}[j] = nx{f}[j]; }}"]
+        K += stores + ["          }", "#pragma unroll", "          for (int j = 0; j < C; ++j) {"]
+        K += [f"            pv{f}[j] = cr{f}[j];" for f in fields] + ["          }"]
         K += ["        }", "      }", "    }", "    put(out_idx);", "  }", "}"]
         return "\n".join(K)
 
@@ -380,22 +394,26 @@ class BatchEmitter:
             K.append(self.emit_reg())
         smem = " + ".join(f"(((size_t)PX * PY * sizeof({el[f]}) + 15) & ~(size_t)15) * 2" for f in fields)
         reg_blocks, reg_launch = [], []
+        regs = REG_ROWS[min(len(fields), 2) - 1]
         if reg:
-            reg_blocks = [f"  if (const int C = xg_tb_reg_{n}(T, ty, tx)) {{",
-                          f"    const size_t bytes = (size_t)64 * 32 * C * sizeof(float) * {len(fields)};"]
-            for c in (2, 4):
+            kinds = [(c, rs) for c in (2, 4) for rs, _ in regs]
+            reg_blocks = [f"  if (const int kind = xg_tb_reg_{n}(T, ty, tx)) {{",
+                          "    const int C = kind & 15, RS = kind >> 4;",
+                          f"    const size_t bytes = (size_t)RS * 8 * 32 * C * sizeof(float) * {len(fields)};"]
+            for c, rs in kinds:
+                reg_blocks.append(f"    if (C == {c} && RS == {rs}) {{")
                 for it in ("int", "int64_t"):
-                    reg_blocks.append(f"    if (C == {c}) XG_TRY(xg_smem_optin(xgk_{n}_tbr<{it}, {c}>, &cap));")
-                reg_blocks.append(f"    if (C == {c}) XG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, "
-                                  f"xgk_{n}_tbr<int, {c}>, 256, bytes));")
+                    reg_blocks.append(f"      XG_TRY(xg_smem_optin(xgk_{n}_tbr<{it}, {c}, {rs}>, &cap));")
+                reg_blocks += [f"      XG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, "
+                               f"xgk_{n}_tbr<int, {c}, {rs}>, 256, bytes));", "    }"]
             reg_blocks += ["    if (per < 1) XG_FAIL(\"temporal blocking: no CTA of the register-block kernel fits an "
                            "SM\");",
                            "    *smem = (int)bytes;", "    *blocks = sms * per;", "    return 0;", "  }"]
-            for c in (2, 4):
+            for c, rs in kinds:
                 for it, cond in (("int", "b.small"), ("int64_t", "!b.small")):
-                    reg_launch.append(f"    {'else ' if reg_launch else ''}if (C == {c} && {cond}) "
-                                      f"xgk_{n}_tbr<{it}, {c}><<<b.blocks, 256, b.smem, s>>>(d, t0, b.nprob, b.total, "
-                                      "dep, b.ty, b.tx, in, out, prev, b.counters + i);")
+                    reg_launch.append(f"    {'else ' if reg_launch else ''}if (kind == {c + 16 * rs} && {cond}) "
+                                      f"xgk_{n}_tbr<{it}, {c}, {rs}><<<b.blocks, 256, b.smem, s>>>(d, t0, b.nprob, "
+                                      "b.total, dep, b.ty, b.tx, in, out, prev, b.counters + i);")
             reg_launch.append("    else")
         H = [f"struct xgbt_{n} {{ const void* desc; int64_t total; int64_t steps; unsigned long long* counters; "
              f"int32_t nprob; int32_t small; int32_t blocks; int32_t T; int32_t ty; int32_t tx; int32_t smem; "
@@ -404,11 +422,12 @@ class BatchEmitter:
              f"  const size_t PX = (size_t)tx + 2 * (size_t)T * {rx}, PY = (size_t)ty + 2 * (size_t)T * {ry};",
              f"  return {smem};",
              "}",
-             "// columns per lane (2 or 4) of the register-block kernel whose box of 64 rows and 64 or 128",
-             "// columns holds a tile and its halo, 0: none does and the shared-memory kernel runs",
+             "// the register-block kernel whose box holds a tile and its halo: columns per lane (2 or 4:",
+             "// 64 or 128 columns) + 16 * rows per warp, 0: none does and the shared-memory kernel runs",
              f"static int xg_tb_reg_{n}(int T, int ty, int tx) {{",
-             f"  if (!{int(reg)} || ty + 2 * T * {ry} > 64 || tx + 2 * T * {rx} > 128) return 0;",
-             f"  return tx + 2 * T * {rx} > 64 ? 4 : 2;",
+             f"  const int rows = ty + 2 * T * {ry}, cols = tx + 2 * T * {rx};",
+             f"  if (!{int(reg)} || rows > {8 * regs[-1][0]} || cols > 128) return 0;",
+             "  return (cols > 64 ? 4 : 2) + 16 * (rows > 64 ? 16 : 8);",
              "}",
              f'extern "C" int xg_batch_tb_blocks_{n}(int block_threads, int T, int ty, int tx, int* smem, '
              f'int* blocks) {{',
@@ -447,8 +466,8 @@ class BatchEmitter:
              "  dim3 block(b.block[0], b.block[1], b.block[2]);",
              f"  const struct xgb_{n}* d = (const struct xgb_{n}*)b.desc;",
              "  const int64_t* t0 = (const int64_t*)(d + b.nprob) + b.nprob;",
-             f"  const int C = xg_tb_reg_{n}(b.T, b.ty, b.tx);",
-             "  (void)C;",
+             f"  const int kind = xg_tb_reg_{n}(b.T, b.ty, b.tx);",
+             "  (void)kind;",
              "  int in = 0;",
              "  for (int64_t i = 0; i < L; ++i) {",
              "    const int dep = (int)(b.steps / L + (i < b.steps % L ? 1 : 0));",

@@ -839,10 +839,10 @@ __device__ __forceinline__ void xg_stv(float* dst, const float* d) {
   if (C == 4) *reinterpret_cast<float4*>(dst) = make_float4(d[0], d[1], d[C - 2], d[C - 1]);
   else *reinterpret_cast<float2*>(dst) = make_float2(d[0], d[1]);
 }
-// A row with its neighbour columns: r[1 .. C] is the lane's, r[0] and r[C + 1] come
-// from the lanes next to it (the first and last lane keep a value of their own).
+// The columns next to a lane's part of a row: the last one of the lane before and the
+// first one of the lane after (the first and last lane get a value of their own).
 template <int C>
-__device__ __forceinline__ void xg_sides(float* r) {
-  r[0] = __shfl_up_sync(0xffffffffu, r[C], 1);
-  r[C + 1] = __shfl_down_sync(0xffffffffu, r[1], 1);
+__device__ __forceinline__ void xg_sides(const float* r, float& west, float& east) {
+  west = __shfl_up_sync(0xffffffffu, r[C - 1], 1);
+  east = __shfl_down_sync(0xffffffffu, r[0], 1);
 }
