@@ -210,6 +210,7 @@ inline int64_t inner_distance(int64_t x, int64_t i, int32_t c, int32_t h, int64_
 struct GraphEntry {
   std::vector<uint8_t> key;
   bool captured = false;
+  bool direct = false;  // one node: a plain launch is cheaper than a graph's (512^2 heat: 8 us against 12 on the GPU)
   cudaGraphExec_t exec = nullptr;
   std::vector<std::array<void*, XG_MAX_LEVELS + 1>> post;  // level[] + scratch per grid
   std::vector<uint8_t> ret;
@@ -660,6 +661,10 @@ int xg_call(xg_entry_fn fn, xg_grid* grids, int ngrids, const void* args, size_t
   }
   g_graphs.splice(g_graphs.begin(), g_graphs, it);
   GraphEntry& e = g_graphs.front();
+  if (e.direct) {
+    lock.unlock();
+    return fn(grids, ngrids, args, nargs, ret, nret, stream);
+  }
   if (!e.captured) {
     XG_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
     int rc = fn(grids, ngrids, args, nargs, ret, nret, stream);
@@ -670,10 +675,13 @@ int xg_call(xg_entry_fn fn, xg_grid* grids, int ngrids, const void* args, size_t
       return rc;
     }
     if (ce != cudaSuccess) return cuda_fail(ce, "cudaStreamEndCapture");
+    size_t nodes = 0;
+    if (cudaGraphGetNodes(graph, nullptr, &nodes) != cudaSuccess) nodes = 0;
     cudaError_t ie = cudaGraphInstantiate(&e.exec, graph, 0);
     cudaGraphDestroy(graph);
     if (ie != cudaSuccess) return cuda_fail(ie, "cudaGraphInstantiate");
     e.captured = true;
+    e.direct = nodes == 1;
     e.post.resize(ngrids);
     for (int i = 0; i < ngrids; ++i) {
       std::copy(grids[i].level, grids[i].level + XG_MAX_LEVELS, e.post[i].begin());

@@ -17,12 +17,19 @@ changed.  ``read(level)`` returns a copy without dirtying anything.
 from __future__ import annotations
 
 import ctypes
+import math
+import struct
 
 import numpy as np
 
 from . import device, runtime
 from .log import Logger
 from .types import GridType, Value, numpy_dtype, parse_annotation
+
+
+# runtime.XGGrid as one record: ndim, levels, shape, level pointers, scratch, mask, aux, aux bytes
+_RECORD = struct.Struct(f"@2i{runtime.XG_MAX_DIM}q{runtime.XG_MAX_LEVELS}Q3Qq")
+assert _RECORD.size == ctypes.sizeof(runtime.XGGrid)
 
 
 class _Level:
@@ -59,7 +66,10 @@ class Grid:
         self._mask = None
         self._scratch = None
         self._aux = None
-        self._nbytes = int(np.prod(self.shape)) * self.numpy_dtype.itemsize
+        self._mask_version = 0
+        self._count = math.prod(self.shape)
+        self._nbytes = self._count * self.numpy_dtype.itemsize
+        self._extents = self.shape + (0,) * (runtime.XG_MAX_DIM - len(self.shape))
 
     # ------------------------------------------------------------ reference API
     @property
@@ -126,12 +136,23 @@ class Grid:
         """Device view of a level as a torch tensor of the grid's shape."""
         if self._sync_device(False):
             device.stream().synchronize()  # uploads done before any stream uses the view
-        dt = device.torch_dtype(self.numpy_dtype)
-        if dt is None:
-            self.logger.dead("tensor() is only available for numeric grids")
         lv = self._levels[level]
-        lv.auth = "dev"  # the caller may write through the view
-        return lv.dev.view(dt)[: int(np.prod(self.shape))].view(self.shape)
+        buf = lv.dev
+        typed = getattr(buf, "_xg_typed", None)
+        # the tensor handed out before stays the one for its buffer unless the caller changed what
+        # it is (its shape, storage or gradient flag): a torch view costs 6 us next to a call
+        if typed is None or typed.shape != self.shape or typed.requires_grad or not typed.is_contiguous() \
+                or typed.data_ptr() != buf.data_ptr():
+            dt = device.torch_dtype(self.numpy_dtype)
+            if dt is None:
+                self.logger.dead("tensor() is only available for numeric grids")
+            # on the buffer's storage, but not a view of the buffer: the buffer keeps the tensor
+            with device.torch().inference_mode(False):
+                typed = device.torch().empty(0, dtype=dt, device=buf.device)
+                typed.set_(buf.untyped_storage(), buf.storage_offset() // self.numpy_dtype.itemsize, self.shape)
+            buf._xg_typed = typed
+        lv.auth = "dev"  # the caller may write through the tensor
+        return typed
 
     def _host(self, level: int, dirty: bool) -> np.ndarray:
         lv = self._levels[level]
@@ -185,28 +206,27 @@ class Grid:
         if self._mask_uploaded is None or not np.array_equal(mask, self._mask_uploaded):
             runtime.check(lib.xg_mask_upload(self._mask, mask.ctypes.data), "mask upload")
             self._mask_uploaded = mask.copy()
+            self._mask_version = lib.xg_mask_version(self._mask)
         self._mask_dirty = False
+
+    def _record(self) -> bytes:
+        """C-ABI view (device pointers) of this grid as the bytes of an ``XGGrid``."""
+        levels = self._levels
+        ptrs = [lv.dev.data_ptr() for lv in levels[: runtime.XG_MAX_LEVELS]]
+        ptrs += [0] * (runtime.XG_MAX_LEVELS - len(ptrs))
+        scratch, aux = self._scratch, self._aux
+        return _RECORD.pack(len(self.shape), len(levels), *self._extents, *ptrs,
+                            scratch.data_ptr() if scratch is not None else 0, self._mask or 0,
+                            aux.data_ptr() if aux is not None else 0, aux.numel() if aux is not None else 0)
 
     def serialize(self) -> runtime.XGGrid:
         """C-ABI view (device pointers) of this grid, cf. xgrid/xgrid/__init__.py:60-68."""
-        g = runtime.XGGrid()
-        g.ndim = len(self.shape)
-        g.levels = len(self._levels)
-        for i, n in enumerate(self.shape):
-            g.shape[i] = n
-        for i, lv in enumerate(self._levels[: runtime.XG_MAX_LEVELS]):
-            g.level[i] = lv.dev.data_ptr()
-        g.scratch = self._scratch.data_ptr() if self._scratch is not None else None
-        g.mask = self._mask
-        g.aux = self._aux.data_ptr() if self._aux is not None else None
-        g.aux_bytes = self._aux.numel() if self._aux is not None else 0
-        return g
+        return runtime.XGGrid.from_buffer_copy(self._record())
 
     def _adopt(self, g: runtime.XGGrid) -> None:
         """Take back the level/scratch exchange that a call made, and mark every
         level as device-current."""
-        if len(self._levels) > runtime.XG_MAX_LEVELS:
-            self.logger.dead(f"at most {runtime.XG_MAX_LEVELS} time levels are supported")
+        self._check_levels()
         bufs = {lv.dev.data_ptr(): lv.dev for lv in self._levels}
         if self._scratch is not None:
             bufs[self._scratch.data_ptr()] = self._scratch
@@ -218,6 +238,16 @@ class Grid:
                 self.logger.dead("internal error: scratch buffer aliases a level")
         for lv, buf in zip(self._levels, new_levels):
             lv.dev = buf  # the host mirror stays attached to the level as staging memory
+            lv.auth = "dev"
+
+    def _check_levels(self) -> None:
+        if len(self._levels) > runtime.XG_MAX_LEVELS:
+            self.logger.dead(f"at most {runtime.XG_MAX_LEVELS} time levels are supported")
+
+    def _written(self) -> None:
+        """Mark every level as device-current after a call that exchanged no buffers."""
+        self._check_levels()
+        for lv in self._levels:
             lv.auth = "dev"
 
     def __del__(self) -> None:

@@ -19,7 +19,7 @@ from .compiler import Compiler, Library
 from .config import get_config
 from .grid import Grid
 from .log import Logger
-from .types import Structure, Void
+from .types import Number, Structure, Void
 
 
 class NativeKernel:
@@ -43,6 +43,11 @@ class NativeKernel:
         self.ret_type = None if isinstance(rt, Void) else rt
         self.scratch_slots = set(self.module.implicit_slots)
         self.nargs = len(self.module.arg_order)
+        self.plain_values = all(isinstance(t, Number) for _, t in self.module.value_args)
+        # (is a grid, name, element, dimension) per argument
+        self.arg_kinds = [(kind == "grid", *((self.module.grid_args[i][0], self.module.grid_args[i][1].element,
+                                              self.module.grid_args[i][1].dimension) if kind == "grid" else (None,) * 3))
+                          for kind, i in self.module.arg_order]
         self.use_graph = self.config.graph and not self.module.device_only
         self.mixed_fn = getattr(self.lib.dylib, f"xg_mixed_{self.module.name}", None)
         if self.mixed_fn is not None:
@@ -136,14 +141,13 @@ class NativeKernel:
         if len(args) != self.nargs:
             raise TypeError(f"this function takes {self.nargs} argument ({len(args)} given)")
         grids, values = [], []
-        for (kind, idx), a in zip(self.module.arg_order, args):
-            if kind == "grid":
+        for (is_grid, name, element, dim), a in zip(self.arg_kinds, args):
+            if is_grid:
                 if not isinstance(a, Grid):
-                    self.logger.dead(f"argument '{self.module.grid_args[idx][0]}' expects an xgrid.Grid")
-                gt = self.module.grid_args[idx][1]
-                if a.element != gt.element or a.dimension != gt.dimension:
-                    self.logger.dead(f"argument '{self.module.grid_args[idx][0]}' expects {gt!r}, "
-                                     f"got {a.typing!r}")
+                    self.logger.dead(f"argument '{name}' expects an xgrid.Grid")
+                if len(a.shape) != dim or (a.element is not element and a.element != element):
+                    gt = self.module.grid_args[len(grids)][1]
+                    self.logger.dead(f"argument '{name}' expects {gt!r}, got {a.typing!r}")
                 grids.append(a)
             else:
                 values.append(a)
@@ -168,20 +172,26 @@ class NativeKernel:
             copied = self._upload_event()
             copied.record(device.stream())
         packed = self.pack(values)
-        arr = (runtime.XGGrid * max(len(grids), 1))(*[g.serialize() for g in grids])
+        sent = b"".join([g._record() for g in grids])
+        buf = bytearray(sent or ctypes.sizeof(runtime.XGGrid))
+        arr = (runtime.XGGrid * max(len(grids), 1)).from_buffer(buf)
         ret = self.ret_type.ctype() if self.ret_type is not None else None
         rc = runtime.load().xg_call(self.fn_ptr, arr, len(grids),
-                                    ctypes.cast(ctypes.byref(packed), ctypes.c_void_p) if values else None,
+                                    ctypes.addressof(packed) if values else None,
                                     ctypes.sizeof(packed) if values else 0,
-                                    ctypes.cast(ctypes.byref(ret), ctypes.c_void_p) if ret is not None else None,
+                                    ctypes.addressof(ret) if ret is not None else None,
                                     ctypes.sizeof(ret) if ret is not None else 0,
                                     device.stream_handle(), 1 if self.use_graph else 0)
         if copied is not None:
             copied.synchronize()
         if rc != 0:
             self.logger.dead(f"kernel '{self.module.name}' failed: {runtime.last_error()}")
-        for g, st in zip(grids, arr):
-            g._adopt(st)
+        if buf == sent:  # no buffers exchanged
+            for g in grids:
+                g._written()
+        else:
+            for g, st in zip(grids, arr):
+                g._adopt(st)
         if ret is None:
             return None
         if isinstance(self.ret_type, Structure):
@@ -195,6 +205,8 @@ class NativeKernel:
         return ev
 
     def pack(self, values: list):
+        if self.plain_values:
+            return self.args_type(*values[: len(self.module.value_args)])
         packed = self.args_type()
         for (name, t), v in zip(self.module.value_args, values):
             setattr(packed, name, t.serialize(v))
@@ -255,16 +267,14 @@ class NativeKernel:
             device.stream().synchronize()
         nprob = len(problems)
         ng = len(self.module.grid_args)
-        arr = (runtime.XGGrid * (nprob * ng))(*[g.serialize() for g in all_grids])
-        packed = b"".join(bytes(self.pack(v)) for v in all_values)
+        records = b"".join([g._record() for g in all_grids])
+        packed = b"".join([bytes(self.pack(v)) for v in all_values])
         stride = ctypes.sizeof(self.args_type) if self.module.value_args else 0
         tiling = self._tiling_key(B["group"])
-        key = (tuple((st.level[k] or 0) for st in arr for k in range(B["depth"])),
-               tuple((st.scratch or 0) if tb else 0 for st in arr),
-               tuple(st.mask or 0 for st in arr), tuple(runtime.load().xg_mask_version(st.mask) for st in arr),
-               packed, tiling, tb[:3] if tb else None)
+        key = (records, tuple([g._mask_version for g in all_grids]), packed, tiling, tb[:3] if tb else None)
         entry = B["desc"].get(key)
         if entry is None:
+            arr = (runtime.XGGrid * (nprob * ng)).from_buffer_copy(records)
             host = ctypes.create_string_buffer(nprob * (B["dsize"] + 16))
             total, maxc, total_tb = ctypes.c_int64(), ctypes.c_int64(), ctypes.c_int64(-1)
             args_buf = ctypes.create_string_buffer(packed, max(len(packed), 1))

@@ -167,12 +167,15 @@ class Structure(Value):
         self.elements_map = dict(self.elements)
         self._ctype = type(f"st{self.name}", (ctypes.Structure,),
                            {"_fields_": [(n, t.ctype) for n, t in self.elements]})
+        self._flat = all(isinstance(t, Number) for _, t in self.elements)
 
     @property
     def ctype(self):
         return self._ctype
 
     def serialize(self, value):
+        if self._flat:  # numbers only: no nested dataclass to unfold
+            return self._ctype(*[getattr(value, f.name) for f in dataclasses.fields(value)])
         return self._ctype(*dataclasses.astuple(value))
 
     def deserialize(self, value):
