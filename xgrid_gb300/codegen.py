@@ -1546,13 +1546,13 @@ class SweepGroupEmitter:
               f"      for (; z + {U} <= z1; z += {U}) {{",
               "        const I zb0 = (I)z * sz;"]
         L += [f"        const I zb{k} = zb{k - 1} + sz;" for k in range(1, U)]
-        if any(1 in zs for zs in win.values()):
+        if win:
             L.append(f"        const int zn = xg_axis(xg_overstep, z + {U}, (int)p.Z);")
         for b, zs in win.items():
             t = self.elem(int(b[1:].split("_")[0]))
             for k in range(U - 1):
                 L.append(f"        const {t} w{b}_{k + 1} = {b}[zb{k + 1} + {c0}];")
-            L.append(f"        const {t} w{b}_{U} = {b}[(I){'zn' if 1 in zs else f'(z + {U - 1})'} * sz + {c0}];")
+            L.append(f"        const {t} w{b}_{U} = {b}[(I)zn * sz + {c0}];")
 
         def wname(k):
             def names_of(b, oz):
@@ -1570,11 +1570,11 @@ class SweepGroupEmitter:
         L += ["      }",
               "      for (; z < z1; ++z) {",
               "        const I zb = (I)z * sz;"]
-        if any(1 in zs for zs in win.values()):
+        if win:
             L.append("        const int zn = xg_axis(xg_overstep, z + 1, (int)p.Z);")
         for b, zs in win.items():
             t = self.elem(int(b[1:].split("_")[0]))
-            L.append(f"        const {t} w{b}_p = {b}[(I){'zn' if 1 in zs else 'z'} * sz + {c0}];")
+            L.append(f"        const {t} w{b}_p = {b}[(I)zn * sz + {c0}];")
         loads, store = plane("        ", "zb", lambda b, oz: f"w{b}_{'m' if oz < 0 else ('p' if oz > 0 else 'c')}", "r")
         L += loads + [store]
         for b in win:
