@@ -137,6 +137,10 @@ int xg_mask_cells(xg_mask* mask, int32_t value, const int64_t** cells, int64_t* 
 /* Number of cells whose mask is nonzero (host-side count, no device work).
  * Runtime helper with no counterpart in the reference. */
 int xg_mask_nonzero(const xg_mask* mask, int64_t* count);
+/* One bit per cell, set where the mask is nonzero: cell x of row z * Y + y is bit
+ * x % 32 of word (z * Y + y) * ceil(X / 32) + x / 32.  Device pointer, owned by the
+ * mask.  Runtime helper with no counterpart in the reference. */
+int xg_mask_bits(xg_mask* mask, const uint32_t** bits);
 /* Tile tables for a tiling of `tile` = {tz, ty, tx} cells (the last tile of
  * each axis absorbs the remainder):  *tile_zero[t] = 1 when every cell of tile
  * t has mask 0;  *csr_off/*csr_cells list the cells of mask `value` grouped by

@@ -573,8 +573,8 @@ class CudaGenerator:
             src.append("  char xg_empty;")
         src.append("};")
         src.append(f"static int xg_fuse_{name} = {1 if self.cfg.fuse else 0};")
-        src.append(f"static int xg_zstage_{name} = 1;  // staged z-walk of mask-free 3-D sweeps (0: register z-walk)")
-        src.append(f"static long long xg_zstage_launches_{name} = 0;  // staged z-walk launches issued by the host")
+        src.append(f"static int xg_zstage_{name} = 1;  // strips and the staged z-walk (0: tiles, register z-walk)")
+        src.append(f"static long long xg_zstage_launches_{name} = 0;  // strip and staged z-walk launches issued by the host")
         src.append(f"static int xg_tloop_{name} = 1;  // several loop iterations per launch where possible (0: one)")
         # launch hook (slab decomposition): called before every single-sweep launch with the
         # launch's site (group * 64 + sweep), so that a caller can refresh halo rows first
@@ -1158,12 +1158,13 @@ def zstage_frame(kname: str, ptype: str, T: str, srcs: list, loads: list, outs: 
     return "\n".join(line for line in K if line)
 
 
-def zstage_launch(kname: str, T: str, nb: int, ind: str, aligned: list, before: list, after: list) -> list:
+def zstage_launch(kname: str, T: str, nb: int, ind: str, aligned: list, before: list, after: list,
+                  only_aligned: bool = False) -> list:
     """Host lines launching ``kname`` (a ``zstage_frame`` kernel) with parameters
     ``p`` on stream ``s`` when its shared memory fits; ``aligned``: the pointers
     (sources and destinations) that must be 16-byte aligned for 16-byte copies;
     ``before`` / ``after`` run around the launch, which ends with ``return 0``.
-    Falls through otherwise."""
+    Falls through otherwise (with ``only_aligned`` also where rows are unaligned)."""
     g = zstage_geometry(T, nb)
     ty, tx = ZSTAGE_TILE
     al = " && ".join(f"((uintptr_t)({a}) & 15) == 0" for a in aligned) or "1"
@@ -1177,7 +1178,7 @@ def zstage_launch(kname: str, T: str, nb: int, ind: str, aligned: list, before: 
          "  int64_t nt = 0;",
          f"  XG_TRY(xg_zstage_chunks(p.Z, p.Y, p.X, {ty}, {tx}, &zlen, &nt));",
          f"  const int vec = (p.X % {g['V']}) == 0 && {al};",
-         "  if (smem <= (size_t)(small ? avail32 : avail64) && nt <= 0x7fffffffLL) {"]
+         f"  if ({'vec && ' if only_aligned else ''}smem <= (size_t)(small ? avail32 : avail64) && nt <= 0x7fffffffLL) {{"]
     L += ["    " + b for b in before]
     L += [f"    if (small) {kname}<int><<<(unsigned)nt, {ZSTAGE_THREADS}, smem, s>>>(p, zlen, vec);",
           f"    else {kname}<int64_t><<<(unsigned)nt, {ZSTAGE_THREADS}, smem, s>>>(p, zlen, vec);",
@@ -1290,6 +1291,10 @@ class SweepGroupEmitter:
             hs.append("  char xg_empty;")
         hs.append("};")
         gen.device_chunks.append("\n".join(hs))
+        splan = self.strip_plan()
+        if splan:
+            from . import strip
+            gen.host_chunks.append("\n".join(strip.apply_lines(self, splan)))
         if self.g.fusable:
             self.emit_fused()
         for j, s in enumerate(self.g.sweeps):
@@ -1299,7 +1304,7 @@ class SweepGroupEmitter:
                 self.emit_bnd_single(j, s)
         lines = [f"static int xgl_{n}_{gid}(xg_grid* G, const struct xgh_{n}_{gid}* h, cudaStream_t s) {{"]
         if self.g.fusable:
-            lines += [f"  if (xg_fuse_{n}) {{",
+            lines += [f"  if (xg_fuse_{n}{f' && !xgl_{n}_{gid}_strips(G)' if splan else ''}) {{",
                       f"    int r = xgl_{n}_{gid}_fused(G, h, s);",
                       "    if (r < 0) return r;",
                       "    if (r > 0) return 0;",
@@ -1380,6 +1385,21 @@ class SweepGroupEmitter:
                   and has_stencil(e) and self.gen.ctype(e) == "double"
                   for s in self.g.sweeps if s.is_main for e in ir.walk(s.stmt.value))
         return 2 if ops >= FP64_HEAVY else BLOCKS_WIDE
+
+    def tile_blocks(self) -> int:
+        """Resident CTAs per SM of the group's tile kernel (the register z-walk keeps
+        several planes in registers)."""
+        mains = [j for j, s in enumerate(self.g.sweeps) if s.is_main]
+        alone = len(self.g.sweeps) == 1 and len(mains) == 1
+        return ZWALK_BLOCKS if alone and self.zmarch_ok(mains, []) else self.min_blocks()
+
+    def strip_plan(self):
+        """Strip plan (``strip.plan``) of the group's main sweep when it is the only one
+        and the first, else None."""
+        from . import strip
+        if any(s.is_main for s in self.g.sweeps[1:]) or not self.g.sweeps[0].is_main:
+            return None
+        return strip.plan(self, 0)
 
     def restrict_locals(self, sweeps) -> list:
         """Kernel-local __restrict__ copies of the buffer pointers: distinct buffer
@@ -1744,7 +1764,7 @@ class SweepGroupEmitter:
                     lo[a] = min(lo[a], ld.offset[a])
                     hi[a] = max(hi[a], ld.offset[a])
         zm = self.zmarch_ok(mains, bnd_phases)
-        blocks = ZWALK_BLOCKS if zm else self.min_blocks()  # the z walk keeps several planes in registers
+        blocks = self.tile_blocks()
         lines = [f"template <typename I> __global__ void __launch_bounds__(256, {blocks}) xgk_{n}_{gid}_{tag}("
                  f"const __grid_constant__ struct xgp_{n}_{gid}_{tag} p) {{"]
         members = [self.g.sweeps[j] for j in list(mains) + list(bnd_phases)]
@@ -1834,7 +1854,7 @@ class SweepGroupEmitter:
             return [f"{indent}const int32_t* tl = xg_tiling_{n}[{gid}];"]
         return [f"{indent}int32_t tl_[6];",
                 f"{indent}const int32_t* tl = xg_tiling_for(xg_tiling_{n}[{gid}], xg_tiling_set_{n}[{gid}], "
-                f"&G[{slot}], tl_);",
+                f"&G[{slot}], {self.tile_blocks()}, tl_);",
                 f"{indent}if (!tl) return -1;"]
 
     def fill_params(self, tag: str, sweeps, dom_slot: int, single=None, indent: str = "  ",
@@ -1917,6 +1937,10 @@ class SweepGroupEmitter:
         zbufs = self.zstage_buffers(j)
         if zbufs:
             self.gen.device_chunks.append(self.zstage_kernel(tag, j, zbufs))
+        from . import strip
+        splan = self.strip_plan() if j == 0 else None
+        if splan:
+            self.gen.device_chunks.extend(strip.kernels(self, tag, j, splan))
         L = [f"static int xgl_{n}_{gid}_{tag}(xg_grid* G, const struct xgh_{n}_{gid}* h, cudaStream_t s) {{"]
         L += self.check_levels(sweeps, s)
         L += self.fill_params(tag, sweeps, s.slot, s)
@@ -1930,6 +1954,8 @@ class SweepGroupEmitter:
             L.append(f"  XG_CUDA(cudaMemcpyAsync(p.{dst}, p.{src}, (size_t)(p.e{s.slot}[0] * p.e{s.slot}[1] * "
                      f"p.e{s.slot}[2]) * sizeof(*p.{dst}), cudaMemcpyDeviceToDevice, s));")
         site = gid * 64 + j
+        swap = [f"{{ void* t_ = G[{s.slot}].level[{s.level}]; G[{s.slot}].level[{s.level}] = "
+                f"G[{s.slot}].scratch; G[{s.slot}].scratch = t_; }}"] if s.implicit else []
         if zbufs:
             # a grid without boundary cells takes the staged z-walk (every tile mask-free)
             L += [f"  if (p.same && xg_zstage_{n}) {{",
@@ -1942,8 +1968,12 @@ class SweepGroupEmitter:
                                [f"if (xg_hook_{n}) XG_TRY(xg_hook_{n}(xg_hook_ctx_{n}, {site}, G, "
                                 f"{len(self.gen.slots)}, s));", f"xg_prof_launch({site}, s);",
                                 f"++xg_zstage_launches_{n};"],
-                               [f"xg_prof_end({site}, s);"])
+                               [f"xg_prof_end({site}, s);"], only_aligned=splan is not None)
             L += ["  }"]
+        if splan:
+            L += [f"  if (const int shape = xgl_{n}_{gid}_strips(G)) {{"]
+            L += strip.launch(self, tag, splan, site, f"G[{s.slot}].mask", "    ")
+            L += ["        " + x for x in [f"++xg_zstage_launches_{n};", *swap, "return 0;"]] + ["      }", "    }", "  }"]
         L += ["  dim3 block(tl[3], tl[4], tl[5]), grid;",
               "  XG_TRY(xg_tile_grid(p.ntx, p.nty, p.ntz, &grid));",
               f"  if (xg_hook_{n}) XG_TRY(xg_hook_{n}(xg_hook_ctx_{n}, {site}, G, {len(self.gen.slots)}, s));",
@@ -1952,10 +1982,7 @@ class SweepGroupEmitter:
               f"  else xgk_{n}_{gid}_{tag}<int64_t><<<grid, block, 0, s>>>(p);",
               "  XG_CUDA(cudaGetLastError());",
               f"  xg_prof_end({site}, s);"]
-        if s.implicit:
-            L.append(f"  {{ void* t_ = G[{s.slot}].level[{s.level}]; G[{s.slot}].level[{s.level}] = "
-                     f"G[{s.slot}].scratch; G[{s.slot}].scratch = t_; }}")
-        L += ["  return 0;", "}"]
+        L += ["  " + x for x in swap] + ["  return 0;", "}"]
         self.gen.host_chunks.append("\n".join(L))
 
     def emit_bnd_single(self, j: int, s) -> None:

@@ -301,6 +301,13 @@ __device__ __forceinline__ int xg_axis(int mode, int c, int n) {
   return c < 0 ? 0 : (c >= n ? n - 1 : c);
 }
 
+// xg_axis for coordinates at most one period outside: one compare and add per side (the
+// remainders of the general form cost instruction cache in unrolled code).
+__device__ __forceinline__ int xg_near(int mode, int c, int n) {
+  if (mode == XG_OVERSTEP_WRAP) return c < 0 ? c + n : (c >= n ? c - n : c);
+  return c < 0 ? 0 : (c >= n ? n - 1 : c);
+}
+
 // Flattened neighbour under "none": -1 outside the allocation.
 __device__ __forceinline__ int64_t xg_flat(int64_t t, int64_t total) { return (t < 0 || t >= total) ? -1 : t; }
 
@@ -345,33 +352,41 @@ static inline int xg_sm_count(int* sms) {
   return 0;
 }
 
-// The tiling of a launch: `cfg` when it was set for the group, else on 2-D grids the
-// default's columns and threads, and a tile count along y (a negative extent) that
-// spreads the cells evenly over the SMs where the default's rows do not.  A sweep that
-// is bound by an SM's FP64 pipe ends with the SM that holds the most tiles: the cost is
-// ceil(tiles / SMs) * (rows per tile + 2), two rows standing for a tile's own tables,
-// barriers and first loads.  The default stays when it costs at most a tenth more (the
-// loops take its 64 rows in whole passes, which a memory-bound sweep feels: 229 against
-// 250 us for the 4097^2 residual launch with 216 rows).  Tiles keep at least 4 rows, so
-// that boundary phases that read the row next to theirs stay inside the tile.
-static inline const int32_t* xg_tiling_for(const int32_t* cfg, int set, const xg_grid* g, int32_t* buf) {
-  if (set || g->ndim != 2) return cfg;
+// The tiling of a launch: `cfg` when it was set for the group, else the default's columns
+// and threads, and a tile count along the slowest axis (a negative extent) that levels the
+// work where the default's does not.
+// 2-D: a sweep that is bound by an SM's FP64 pipe ends with the SM that holds the most
+// tiles: the cost is ceil(tiles / SMs) * (rows per tile + 2), two rows standing for a
+// tile's own tables, barriers and first loads.  Tiles keep at least 4 rows, so that
+// boundary phases that read the row next to theirs stay inside the tile.
+// 3-D: a tile's CTA walks all of its planes, so a launch takes whole rounds of the `blocks`
+// CTAs an SM holds: ceil(tiles / (SMs * blocks)) * (planes per tile + 2), at least 8 planes.
+// The default stays when it costs at most a tenth more (on 2-D grids the loops take its
+// 64 rows in whole passes, which a memory-bound sweep feels: 229 against 250 us for the
+// 4097^2 residual launch with 216 rows).
+static inline const int32_t* xg_tiling_for(const int32_t* cfg, int set, const xg_grid* g, int blocks, int32_t* buf) {
+  if (set || g->ndim < 2) return cfg;
   int sms = 0;
   if (xg_sm_count(&sms) != 0) return NULL;
   const xg_ext e = xg_extent(g);
-  const int64_t ntx = xg_tiles_along(e.x, cfg[2]), n0 = xg_tiles_along(e.y, cfg[1]);
-  int64_t best = -1, first = -1, count = n0;
-  for (int64_t n = n0; n == n0 || (n <= e.y / 4 && n <= n0 + 256); ++n) {
-    const int64_t cost = ((n * ntx + sms - 1) / sms) * ((e.y + n - 1) / n + 2);
-    if (first < 0) first = cost;
-    if (best < 0 || cost < best) {
-      best = cost;
+  const int flat = g->ndim == 2;
+  const int64_t len = flat ? e.y : e.z;
+  const int64_t per = xg_tiles_along(e.x, cfg[2]) * (flat ? 1 : xg_tiles_along(e.y, cfg[1]));
+  const int64_t slots = flat ? sms : (int64_t)sms * blocks;
+  const int64_t n0 = xg_tiles_along(len, cfg[flat ? 1 : 0]);
+  const int64_t n1 = flat ? n0 : 1, nmax = len / (flat ? 4 : 8);
+  int64_t best = -1, count = n0;
+  auto cost = [&](int64_t n) { return ((n * per + slots - 1) / slots) * ((len + n - 1) / n + 2); };
+  for (int64_t n = n1; n <= nmax && n <= n1 + 256; ++n) {
+    const int64_t c = cost(n);
+    if (best < 0 || c < best) {
+      best = c;
       count = n;
     }
   }
-  if (10 * first <= 11 * best || count > 65535) return cfg;
+  if (best < 0 || 10 * cost(n0) <= 11 * best || count > 65535) return cfg;
   memcpy(buf, cfg, 6 * sizeof(int32_t));
-  buf[1] = -(int32_t)count;
+  buf[flat ? 1 : 0] = -(int32_t)count;
   return buf;
 }
 
@@ -383,6 +398,24 @@ struct xg_tile {
   int64_t t;
 };
 
+// Even split of n cells into nt tiles: [lo, hi) of tile i, lo = floor(i * n / nt), in
+// 32-bit arithmetic (64-bit divisions took 400 of the 590 instructions of a warp of the
+// 4096^2 transport sweep).
+__device__ __forceinline__ void xg_even_range(unsigned n, unsigned nt, unsigned i, int* lo, int* hi) {
+  unsigned a = 0, b = n;
+  if (nt > 1) {
+    const unsigned q = n / nt, r = n - q * nt;  // floor(i n / nt) = i q + floor(i r / nt)
+    a = i * q;
+    b = a + q;
+    if (r) {
+      a += nt < 65536u ? i * r / nt : (unsigned)((uint64_t)i * r / nt);
+      b += nt < 65536u ? (i + 1) * r / nt : (unsigned)((uint64_t)(i + 1) * r / nt);
+    }
+  }
+  *lo = (int)a;
+  *hi = (int)b;
+}
+
 // Tile (iz, iy, ix): along z and y, tile i of nt covers [i * n / nt, (i + 1) * n / nt)
 // (even split, tiles differ by at most one cell); along x, tiles of tx cells with the
 // last one absorbing the remainder (columns stay aligned to the warps).
@@ -392,10 +425,8 @@ __device__ __forceinline__ xg_tile xg_tile_even(int64_t iz, int64_t iy, int64_t 
   T.t = (iz * nty + iy) * ntx + ix;
   T.x0 = (int)(ix * tx);
   T.x1 = (ix == ntx - 1) ? (int)X : (int)((ix + 1) * tx);
-  T.y0 = (int)(iy * Y / nty);
-  T.y1 = (int)((iy + 1) * Y / nty);
-  T.z0 = (int)(iz * Z / ntz);
-  T.z1 = (int)((iz + 1) * Z / ntz);
+  xg_even_range((unsigned)Y, (unsigned)nty, (unsigned)iy, &T.y0, &T.y1);
+  xg_even_range((unsigned)Z, (unsigned)ntz, (unsigned)iz, &T.z0, &T.z1);
   return T;
 }
 
@@ -733,6 +764,32 @@ static inline int xg_zstage_chunks(int64_t Z, int64_t Y, int64_t X, int ty, int 
   if (best_len > 0x7fffffffLL) XG_FAIL("staged z-walk: chunk of %lld planes", (long long)best_len);
   *zlen = (int)best_len;
   *nt = ncb * ((Z + best_len - 1) / best_len);
+  return 0;
+}
+
+// Chunks of a strip launch (strip.py) over A planes (rows of 2-D grids) of NY rows (1 on
+// 2-D grids) of X columns: strips of `w` columns by `r` rows, and the chunk length along
+// the slowest axis that minimises ceil(warps / resident warps) * (planes per chunk + 3),
+// three planes standing for a chunk's first loads; chunks hold at least 8 planes.  *nw
+// receives the warp count.
+static inline int xg_strip_chunks(int64_t A, int64_t NY, int64_t X, int w, int r, int warps_per_sm, int* alen,
+                                  int64_t* nsx, int64_t* nsy, int64_t* nw) {
+  int sms = 0;
+  XG_TRY(xg_sm_count(&sms));
+  const int64_t nx = (X + w - 1) / w, ny = (NY + r - 1) / r, slots = (int64_t)sms * warps_per_sm;
+  int64_t best = -1, len = A;
+  for (int64_t c = 1; c <= (A / 8 > 1 ? A / 8 : 1) && c <= 4096; ++c) {
+    const int64_t l = (A + c - 1) / c, chunks = (A + l - 1) / l;
+    const int64_t cost = ((nx * ny * chunks + slots - 1) / slots) * (l + 3);
+    if (best < 0 || cost < best) {
+      best = cost;
+      len = l;
+    }
+  }
+  *alen = (int)len;
+  *nsx = nx;
+  *nsy = ny;
+  *nw = nx * ny * ((A + len - 1) / len);
   return 0;
 }
 

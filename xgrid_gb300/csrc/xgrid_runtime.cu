@@ -117,8 +117,11 @@ struct xg_mask {
   std::map<TileKey, Tiles> tiles;
   std::map<BoxKey, Boxes> boxes;
   std::map<std::string, int> local_cache;
+  uint32_t* bits = nullptr;  // one bit per cell (nonzero mask), rows padded to whole words
 
   void release_tables() {
+    cudaFree(bits);
+    bits = nullptr;
     for (auto& kv : cells_dev) cudaFree(kv.second);
     cells_dev.clear();
     for (auto& kv : tiles) {
@@ -331,6 +334,22 @@ int xg_mask_nonzero(const xg_mask* m, int64_t* count) {
   int64_t n = 0;
   for (const auto& kv : m->cells) n += static_cast<int64_t>(kv.second.size());
   *count = n;
+  return 0;
+}
+
+int xg_mask_bits(xg_mask* m, const uint32_t** bits) {
+  if (!m || !bits) return fail("xg_mask_bits: null argument");
+  if (!m->bits) {
+    const int64_t words = (m->ext[2] + 31) / 32;
+    std::vector<uint32_t> w(static_cast<size_t>(m->ext[0] * m->ext[1] * words), 0u);
+    for (const auto& kv : m->cells)
+      for (int64_t c : kv.second) {
+        const int64_t x = c % m->ext[2];
+        w[static_cast<size_t>(c / m->ext[2] * words + x / 32)] |= 1u << (x & 31);
+      }
+    if (upload(w, &m->bits)) return -1;
+  }
+  *bits = m->bits;
   return 0;
 }
 
