@@ -41,8 +41,8 @@ Backend options (new keywords, all optional):
 * ``loop_temporal``: iterations per launch of an in-place loop of that kind on
   2-D grids under overstep "none" whose level fits in a quarter of L2 (boxes of
   the grid staged in shared memory with a halo of that many cells, recomputed per
-  iteration; ``xgrid_gb300.tloop``; default 3, the fastest of 2/3/4 measured on a
-  GB300 for the 1025^2 cavity); 0 or 1: one launch per iteration.  Same arithmetic per cell, same bits; applies
+  iteration; ``xgrid_gb300.tloop``); 0 or 1: one launch per iteration; left at its
+  default, 2 to 6 by the grid's size.  Same arithmetic per cell, same bits; applies
   only when the box check proves every read exact, else one launch per
   iteration.
 * ``fail_waits``: for testing only.  Compile modules whose give-up waits cannot
@@ -74,6 +74,13 @@ _MIXED = (None, "fp32", "fp16", "bf16")
 MIXED_ROWS = (4, 8)
 
 
+class _Default(int):
+    """A keyword's default value, told apart from the same number given by the caller."""
+
+
+LOOP_TEMPORAL = _Default(3)
+
+
 @dataclasses.dataclass
 class Configuration:
     parallel: bool
@@ -96,6 +103,7 @@ class Configuration:
     persistent: bool = False
     fail_waits: bool = False
     loop_temporal: int = 3
+    loop_auto: bool = False  # loop_temporal was left at its default: the depth by the grid's size
 
     def __repr__(self) -> str:
         return repr(dataclasses.asdict(self))
@@ -129,7 +137,7 @@ def init(*, parallel: bool = True, cc: list = ["gcc", "clang"], cacheroot: str =
          exact: bool = True, mixed: Optional[str] = None, graph: bool = True,
          fuse: bool = True, divisor: bool = True, mixed_every: int = 0, autotune: bool = True,
          mixed_temporal: int = 8, mixed_rows: int = 8, int_adds: int = 0, persistent: bool = False,
-         fail_waits: bool = False, loop_temporal: int = 3) -> None:
+         fail_waits: bool = False, loop_temporal: int = LOOP_TEMPORAL) -> None:
     """Set the global configuration (same keywords as the reference plus GPU options)."""
     global _config
     if sys.version_info < (3, 10):
@@ -153,5 +161,5 @@ def init(*, parallel: bool = True, cc: list = ["gcc", "clang"], cacheroot: str =
     _config = Configuration(parallel, list(cc), cacheroot, comment, overstep, opt_level,
                             precision, exact, mixed, graph, fuse, divisor, int(mixed_every), bool(autotune),
                             int(mixed_temporal), int(mixed_rows), int(int_adds), bool(persistent),
-                            bool(fail_waits), int(loop_temporal))
+                            bool(fail_waits), int(loop_temporal), isinstance(loop_temporal, _Default))
     logger.info(f"initialized with configuration: {_config}")

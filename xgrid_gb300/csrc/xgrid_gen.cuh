@@ -627,6 +627,24 @@ __device__ __forceinline__ void xg_tile_done(unsigned* flags, int64_t t, unsigne
   }
 }
 
+// Cycles per iteration of a launch of th iterations on nb boxes of r core rows and w
+// columns, per_sm of them resident per SM: the boxes of the busiest SM share its FP64
+// pipe (half a cycle per cell and operation), a box alone takes its own latency, and a launch costs a ramp,
+// the staging and the write-back of every round of boxes.  The constants are fitted to
+// cavity steps (us, against 3 iterations in boxes that minimise cells per CTA slot):
+// 129^2 144 -> 109, 257^2 165 -> 151, 513^2 270 -> 269, 700^2 739 -> 682, 1025^2 722 -> 698,
+// 1200^2 1786 -> 1703, 1500^2 2564 -> 2472.
+static inline double xg_boxes_cost(int64_t nb, int sms, int per_sm, int nt, int ops, int r, int w, int th) {
+  const int64_t most = (nb + sms - 1) / sms, rounds = (most + per_sm - 1) / per_sm;
+  double t = 6000;
+  for (int k = 1; k <= th; ++k) {
+    const double cells = (double)(r + 2 * th - 2 * k) * w;  // a warp's 32 columns cost the same with halo lanes off
+    const double pipe = most * cells * (0.6 * ops + 0.2), own = rounds * (700 + ceil(cells / nt) * 800);
+    t += pipe > own ? pipe : own;
+  }
+  return (t + 2500 * rounds) / th;
+}
+
 // ---------------------------------------------------------------------------
 // Power-of-two storage scales of 16-bit fields.  For a field whose largest
 // magnitude is m, xg_scale_exp(m, A) = A - floor(log2 m) (clamped to the normal

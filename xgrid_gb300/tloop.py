@@ -21,8 +21,9 @@ up to ``TH`` iterations of the group on *boxes*:
 
 Only grids whose level takes at most a quarter of L2 use it: larger ones stream
 from HBM, where the launch ramp is small against a sweep and the halo work is
-not repaid (1025^2 FP64 cavity: 0.854 -> 0.761 ms per step with 3 iterations per
-launch; 4097^2: 10.08 -> 10.26 ms).
+not repaid (4097^2 FP64 cavity: 10.08 -> 10.26 ms per step with 3 iterations per launch).
+Iterations per launch and box shape come from a cost model (``xg_boxes_cost``) unless the
+caller fixed the iterations.
 
 Every cell gets the same operations in the same order as in the one-iteration
 kernel, so the results are bit-identical.  The halo of ``TH`` cells keeps the
@@ -36,9 +37,10 @@ from __future__ import annotations
 
 from . import analysis
 
-THREADS = 256
+THREADS = 512
+DEEPEST = 6  # iterations of a launch that the depth rule may take (8: its boxes fail the check on small grids)
 SITE = 57  # profiling site of the launch within its group
-MIN_BLOCKS = 4  # resident CTAs per SM asked of ptxas (the boxes of a wave are sized for four)
+MIN_BLOCKS = 2  # resident CTAs per SM asked of ptxas (4 of 256 threads: 4 to 10 % slower from 513^2 on)
 
 
 def plan(em) -> dict | None:
@@ -86,6 +88,25 @@ def plan(em) -> dict | None:
     return {"slot": slot, "level": level, "main_offs": main_offs, "phases": phases}
 
 
+def fp64_ops(em, sweep) -> str:
+    """Host expression of the FP64 operations per cell of a sweep: products and quotients
+    by launch constants cost what their parameter says (none for powers of two)."""
+    from . import ir
+    from .codegen import has_stencil
+    n, terms = 0, []
+    for e in ir.walk(sweep.stmt.value):
+        if not isinstance(e, ir.Binary) or not has_stencil(e) or em.gen.ctype(e) != "double":
+            continue
+        if id(e) in em.div_map:
+            k = f"h->{em.div_map[id(e)].name}"
+            terms.append(f"({k}.rz.p2 ? 0 : ({k}.two ? 2 : 4))")
+        elif id(e) in em.mul_map:
+            terms.append(f"(h->{em.mul_map[id(e)][0].name}.p2 ? 0 : 1)")
+        elif not e.operator.is_compare() and not e.operator.is_logic():
+            n += 1
+    return " + ".join([str(n)] + terms)
+
+
 def emit(em, th: int) -> None:
     """Device kernel and host launcher ``xgl_<name>_<gid>_tloop(G, h, K, s)`` (1:
     ran the K iterations, 0: not applicable, negative: error)."""
@@ -102,7 +123,7 @@ def emit(em, th: int) -> None:
     T = em.elem(slot)
     src = em.bname((slot, level, sweeps[0].read_version_of_target))
     dst = em.bname((slot, level, sweeps[0].write_version))
-    extra = ["int32_t cy, cx, nby, nbx, iters", "const int32_t* m", "const uint8_t* bzero"]
+    extra = ["int32_t cy, cx, nby, nbx, iters, th", "const int32_t* m", "const uint8_t* bzero"]
     for j, _, _ in pl["phases"]:
         extra += [f"const int32_t* bo{j}", f"const int32_t* bl{j}"]
     em.gen.device_chunks.append(em.params_struct("tl", sweeps, extra))
@@ -128,7 +149,8 @@ def emit(em, th: int) -> None:
 
     K = [f"template <typename I, int BX> __global__ void __launch_bounds__({THREADS}, {MIN_BLOCKS}) "
          f"xgk_{n}_{gid}_tl(const __grid_constant__ struct xgp_{n}_{gid}_tl p) {{",
-         f"  constexpr int TH = {th}, NT = {THREADS};",
+         f"  constexpr int NT = {THREADS};",
+         "  const int TH = p.th;",
          "  extern __shared__ __align__(16) unsigned char xg_tl_raw[];",
          "  const int BY = p.cy + 2 * TH, NB = BY * BX;",
          f"  {T}* S0 = ({T}*)xg_tl_raw;",
@@ -153,8 +175,9 @@ def emit(em, th: int) -> None:
          "  __syncthreads();",
          f"  {T}* Sa = S0;",
          f"  {T}* Sb = S1;",
-         "  for (int k = 1; k <= p.iters; ++k) {",
-         "    // cells at distance >= k from the box edge are exact after iteration k",
+         "  // cells at distance >= j from the box edge are exact after iteration j; a launch of fewer",
+         "  // iterations than TH leaves out the outermost rings that none of them needs",
+         "  for (int k = 1 + TH - p.iters; k <= TH; ++k) {",
          ]
     K += ["    for (int l = tid; l < NB; l += NT) {",
           "      const int ly = l / BX, lx = l % BX;",
@@ -202,9 +225,8 @@ def emit(em, th: int) -> None:
     def arr(name, typ, xs):
         return [f"  static const {typ} {name}[] = {{{', '.join(str(v) for v in xs) if xs else '0'}}};"]
     site = gid * 64 + SITE
-    bxs = (64, 96, 128)
+    bxs = (32, 64, 96, 128)
     L = [f"static int xgl_{n}_{gid}_tloop(xg_grid* G, const struct xgh_{n}_{gid}* h, int64_t K, cudaStream_t s) {{",
-         f"  constexpr int TH = {th};",
          f"  if (!xg_tloop_{n} || G[{slot}].ndim != 2) return 0;"]
     L += em.check_levels(sweeps)
     L += em.fill_params("tl", sweeps, slot)
@@ -221,32 +243,46 @@ def emit(em, th: int) -> None:
           "  }"]
     L += arr("mo", "int32_t", [v for t in mo for v in t]) + arr("vals", "int32_t", vals)
     L += arr("nof", "int32_t", nof) + arr("offs", "int32_t", offs)
-    L += ["  // core of a box: the (rows, box width) pair whose busiest SM has the fewest box cells",
-          "  static int64_t key_y = -1, key_x = -1;",
-          "  static int cy = 0, bx = 0;",
-          "  if (key_y != p.Y || key_x != p.X) {",
-          "    int dev = 0, sms = 0;",
-          "    XG_CUDA(cudaGetDevice(&dev));",
-          "    XG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));",
-          "    int64_t best = -1;",
-          f"    for (int w : {{{', '.join(str(v) for v in bxs)}}}) {{",
-          "      const int cx = w - 2 * TH;",
-          "      for (int r = 4; r <= 40; ++r) {",
-          f"        const size_t smem = (size_t)(r + 2 * TH) * w * (2 * sizeof({T}) + sizeof(int32_t));",
-          "        const int per_sm = (int)((228 * 1024) / (smem + 1024)) < 4 ? (int)((228 * 1024) / (smem + 1024)) : 4;",
-          "        if (per_sm < 1) continue;",
-          "        const int64_t nb = ((p.Y + r - 1) / r) * ((p.X + cx - 1) / cx);",
-          "        const int64_t slots = (int64_t)sms * per_sm;",
-          "        const int64_t cost = ((nb + slots - 1) / slots) * (int64_t)(r + 2 * TH) * w;",
-          "        if (best < 0 || cost < best) { best = cost; cy = r; bx = w; }",
-          "      }",
+    auto = gen.cfg.loop_auto
+    L += ["  // iterations per launch, core rows and box width with the least time per iteration" +
+          ("; at the\n  // configured depth where the mask does not allow the one that came out" if auto else ""),
+          f"  const int ops = {fp64_ops(em, sweeps[0])};  // FP64 operations per cell of the main sweep",
+          f"  constexpr int TH = {th};  // the configured depth" + (f"; the rule takes 2 to {DEEPEST}" if auto else ""),
+          f"  constexpr int NC = {2 if auto else 1}, lo_th[] = {{{'2, TH' if auto else 'TH'}}}, "
+          f"hi_th[] = {{{f'{DEEPEST}, TH' if auto else 'TH'}}};",
+          "  struct shape { int cy, bx, th; };",
+          "  static thread_local int64_t key_y = -1, key_x = -1;",
+          "  static thread_local int key_ops = -1;",
+          "  static thread_local struct shape kept[NC];",
+          "  if (key_y != p.Y || key_x != p.X || key_ops != ops) {",
+          "    int sms = 0;",
+          "    XG_TRY(xg_sm_count(&sms));",
+          "    for (int c = 0; c < NC; ++c) {",
+          "      double best = -1;",
+          "      for (int t = lo_th[c]; t <= hi_th[c]; ++t)",
+          f"        for (int w : {{{', '.join(str(v) for v in bxs)}}}) {{",
+          "          const int cx = w - 2 * t;",
+          "          for (int r = 4; cx >= 8 && r <= 64; ++r) {",
+          f"            const size_t smem = (size_t)(r + 2 * t) * w * (2 * sizeof({T}) + sizeof(int32_t));",
+          f"            const int fit = (int)((228 * 1024) / (smem + 1024)), per_sm = fit < {MIN_BLOCKS} ? fit : {MIN_BLOCKS};",
+          "            if (per_sm < 1) continue;",
+          "            const int64_t nb = ((p.Y + r - 1) / r) * ((p.X + cx - 1) / cx);",
+          f"            const double cost = xg_boxes_cost(nb, sms, per_sm, {THREADS}, ops, r, w, t);",
+          "            if (best < 0 || cost < best) { best = cost; kept[c] = {r, w, t}; }",
+          "          }",
+          "        }",
           "    }",
-          "    key_y = p.Y; key_x = p.X;",
+          "    key_y = p.Y; key_x = p.X; key_ops = ops;",
           "  }",
-          "  const int32_t core[3] = {1, cy, bx - 2 * TH}, halo[3] = {0, TH, TH}, shrink[3] = {0, 1, 1};",
-          "  int ok = 0;",
-          f"  XG_TRY(xg_mask_box_check(G[{slot}].mask, core, halo, shrink, TH, {len(mo)}, mo, {len(vals)}, vals, nof, "
+          "  int cy = 0, bx = 0, D = 0, ok = 0;",
+          "  int32_t core[3] = {1, 1, 1}, halo[3] = {0, 0, 0};",
+          "  const int32_t shrink[3] = {0, 1, 1};",
+          "  for (int c = 0; c < NC && !ok; ++c) {",
+          "    cy = kept[c].cy; bx = kept[c].bx; D = kept[c].th;",
+          "    core[1] = cy; core[2] = bx - 2 * D; halo[1] = halo[2] = D;",
+          f"    XG_TRY(xg_mask_box_check(G[{slot}].mask, core, halo, shrink, D, {len(mo)}, mo, {len(vals)}, vals, nof, "
           "offs, &ok));",
+          "  }",
           "  if (!ok) return 0;",
           "  int64_t nb = 0;",
           f"  XG_TRY(xg_mask_boxes(G[{slot}].mask, core, halo, 0, &p.bzero, NULL, NULL, &nb));"]
@@ -256,9 +292,9 @@ def emit(em, th: int) -> None:
           "  //  several may come from an entry that may not build them)",
           "  if (K < 2 || nb > 0x7fffffffLL) return 0;",
           f"  p.m = xg_mask_device(G[{slot}].mask);",
-          "  p.cy = cy; p.cx = bx - 2 * TH;",
+          "  p.cy = cy; p.cx = bx - 2 * D; p.th = D;",
           "  p.nby = (int32_t)((p.Y + p.cy - 1) / p.cy); p.nbx = (int32_t)((p.X + p.cx - 1) / p.cx);",
-          f"  const size_t smem = (size_t)(cy + 2 * TH) * bx * (2 * sizeof({T}) + sizeof(int32_t));",
+          f"  const size_t smem = (size_t)(cy + 2 * D) * bx * (2 * sizeof({T}) + sizeof(int32_t));",
           "  const bool small = xg_small_index(p.Z, p.Y, p.X);"]
     for w in bxs:
         for it, tag in (("int", "32"), ("int64_t", "64")):
@@ -266,7 +302,7 @@ def emit(em, th: int) -> None:
                   f"  if (avail_{w}_{tag} < 0) XG_TRY(xg_smem_optin(xgk_{n}_{gid}_tl<{it}, {w}>, &avail_{w}_{tag}));",
                   f"  if (bx == {w} && smem > (size_t)avail_{w}_{tag}) return 0;"]
     L += ["  for (int64_t done = 0; done < K;) {",
-          "    p.iters = (int32_t)(K - done < TH ? K - done : TH);",
+          "    p.iters = (int32_t)(K - done < D ? K - done : D);",
           f"    p.{src} = ({T}*)G[{slot}].level[{level}];",
           f"    p.{dst} = ({T}*)G[{slot}].scratch;",
           f"    xg_prof_launch({site}, s);"]
