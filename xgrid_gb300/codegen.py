@@ -941,12 +941,14 @@ def unsafe_int_div(e) -> bool:
                and isinstance(n.type, Integer) for n in ir.walk(e))
 
 
-def zstage_geometry(T: str, nb: int) -> dict:
-    """Shape of a staged z-walk CTA for element type ``T`` and ``nb`` staged
-    buffers: V cells per 16-byte vector, NTX x NTY threads, RY rows per thread,
+def zstage_geometry(T: str, nb: int, nacc: int = 0) -> dict:
+    """Shape of a staged z-walk CTA for element type ``T``, ``nb`` staged
+    buffers and ``nacc`` accumulated outputs: V cells per 16-byte vector, NTX x NTY threads, RY rows per thread,
     plane rows of PX = TX + 2V elements (cell x0 at column V, halo at V - 1 and
     V + TX), D planes beyond the next one in flight (one when three or more
-    buffers share the ring, so that three CTAs fit on an SM)."""
+    buffers share the ring, so that three CTAs fit on an SM).  ``acc`` bytes after the
+    ring hold D + 1 planes of every thread's old values of accumulated outputs, 0 where
+    they would cost a resident CTA."""
     ty, tx = ZSTAGE_TILE
     size = 8 if T == "double" else 4
     v = 16 // size
@@ -964,8 +966,11 @@ def zstage_geometry(T: str, nb: int) -> dict:
     # D + 3 slots: planes z - 1, z, z + 1 and D in flight, a second barrier per plane before a
     # slot is refilled; one slot more lets the plane's first barrier cover the refill
     slots = d + 4 if ZSTAGE_ONE_BARRIER and fit(d + 4) == fit(d + 3) else d + 3
+    acc = nacc * (d + 1) * (ty // nty) * ZSTAGE_THREADS * 16
+    if fit(slots) * (slots * plane + acc + 1024) > 228 * 1024:
+        acc = 0
     return {"V": v, "NTX": ntx, "NTY": nty, "RY": ty // nty, "D": d, "PX": px, "TY": ty, "TX": tx,
-            "R": slots, "smem": slots * plane, "size": size, "blocks": fit(slots)}
+            "R": slots, "smem": slots * plane + acc, "acc": acc, "size": size, "blocks": fit(slots)}
 
 
 def zstage_frame(kname: str, ptype: str, T: str, srcs: list, loads: list, outs: list) -> str:
@@ -974,7 +979,10 @@ def zstage_frame(kname: str, ptype: str, T: str, srcs: list, loads: list, outs: 
     every source buffer, block plus a one-cell halo (wrapped or clamped), through
     a ring of shared-memory slots with cp.async, D planes beyond the next one in
     flight; 16-byte copies where the block's rows and halo lie inside the grid
-    and ``vec`` says the rows are 16-byte aligned, element copies otherwise.
+    and ``vec`` says the rows are 16-byte aligned, element copies otherwise.  Two
+    instantiations by ``vec``: unaligned rows keep the element copies' offsets in
+    registers and leave out what lies beyond the grid's last halo cells (rollout of 20
+    steps at 203 x 245 x 307: 5450 -> 5110 us; offsets worked out per copy before).
     Every thread owns a 16-byte vector of V consecutive cells in RY rows: per
     plane it reads each needed row of each buffer as one vector from shared
     memory, plus the single cells left and right of it, and computes its V cells
@@ -985,15 +993,37 @@ def zstage_frame(kname: str, ptype: str, T: str, srcs: list, loads: list, outs: 
     ``outs``: (destination pointer, value, guard or None, accumulate) -- the cell
     value (an expression of the load variables) is stored, or added to the
     destination's value when ``accumulate``; a guard skips the output when it
-    is null.  The parameter struct has Z, Y, X."""
-    g = zstage_geometry(T, len(srcs))
+    is null.  The old values of accumulated outputs are copied a plane ahead, by
+    the thread that will add to them, to its own place in shared memory: loaded
+    where they are added, each plane waited for HBM once more (256^3 FP32 rollout of
+    20 steps and its gradients: 3331 -> 3169 us).
+    The parameter struct has Z, Y, X."""
+    accs = [o for o, (_, _, _, add) in enumerate(outs) if add]
+    g = zstage_geometry(T, len(srcs), len(accs))
     V, NTX, NTY, RY, D, PX, TY, TX, R = (g[k] for k in ("V", "NTX", "NTY", "RY", "D", "PX", "TY", "TX", "R"))
 
     VT = "double2" if T == "double" else "float4"
     nb = len(srcs)
     comp = "xyzw"
-    K = [f"template <typename I> __global__ void __launch_bounds__({ZSTAGE_THREADS}, {g['blocks']}) "
-         f"{kname}(const __grid_constant__ {ptype} p, const int zlen, const int vec) {{",
+    old = []
+    if g["acc"]:  # the copies of plane q join the group of the planes staged with them: landed D planes later
+        old = [f"  {VT}* const olds = ({VT}*)(ring + R * NB * PL) + tid;  // [D + 1][outputs][{RY}][NT]",
+               "  auto old_planes = [&](int q) {",
+               "    if (vec && q < z1 && x < (int)p.X) {",
+               "#pragma unroll",
+               f"      for (int i = 0; i < {RY}; ++i) {{",
+               f"        const int y = y0 + ty_t + i * {NTY};",
+               "        const I gb = (I)q * sz + (I)y * sy + (I)x;",
+               f"        {VT}* const to = olds + (((q - z0) % (D + 1)) * {len(accs)} * {RY} + i) * NT;"]
+        for a, o in enumerate(accs):
+            dst, _, guard, _ = outs[o]
+            cond = "y < (int)p.Y" + (f" && {guard}" if guard else "")
+            old.append(f"        if ({cond}) xg_cp_async16(({T}*)(to + {a * RY} * NT), {dst} + gb);")
+        old += ["      }", "    }", "  };",
+                "#pragma unroll",
+                "  for (int q = 0; q < D; ++q) old_planes(z0 + q);"]
+    K = [f"template <typename I, bool vec> __global__ void __launch_bounds__({ZSTAGE_THREADS}, {g['blocks']}) "
+         f"{kname}(const __grid_constant__ {ptype} p, const int zlen) {{",
          f"  constexpr int TY = {TY}, TX = {TX}, V = {V}, NTX = {NTX}, NT = {ZSTAGE_THREADS}, D = {D};",
          f"  constexpr int PX = {PX}, PY = TY + 2, PL = PY * PX, R = {R}, NB = {nb};",
          "  constexpr int CR = TX / V + 2, KC = (PY * CR + NT - 1) / NT;  // copies per row and per thread",
@@ -1029,12 +1059,41 @@ def zstage_frame(kname: str, ptype: str, T: str, srcs: list, loads: list, outs: 
          "      }",
          "    }",
          "  }",
+         "  // rows that are not 16-byte aligned: element copies, lane by lane along the rows of each warp;",
+         "  // columns and rows beyond the halo of the grid's last cells are left out",
+         "  constexpr int NW = NT / 32, RW = (PY + NW - 1) / NW, CE = (TX + 2 + 31) / 32;",
+         "  const int lane = tid % 32, warp = tid / 32;",
+         "  I yo[RW];",
+         "  int xo[CE];",
+         "  if constexpr (!vec) {",
+         "#pragma unroll",
+         "    for (int j = 0; j < RW; ++j) {",
+         "      const int r = warp + NW * j;",
+         "      yo[j] = r < PY && y0 - 1 + r <= (int)p.Y ? (I)xg_axis(xg_overstep, y0 - 1 + r, (int)p.Y) * sy : (I)-1;",
+         "    }",
+         "#pragma unroll",
+         "    for (int k = 0; k < CE; ++k) {",
+         "      const int c = lane + 32 * k;",
+         "      xo[k] = c < TX + 2 && x0 - 1 + c <= (int)p.X ? xg_axis(xg_overstep, x0 - 1 + c, (int)p.X) : -1;",
+         "    }",
+         "  }",
          f"  const {T}* const src[NB] = {{{', '.join(srcs)}}};",
          "  auto stage = [&](int q) {  // plane q into its ring slot (no copies for q beyond the chunk)",
          "    if (q <= z1) {",
          "      const I zb = (I)xg_axis(xg_overstep, q, (int)p.Z) * sz;",
          f"      {T}* const slot = ring + ((q - z0 + 1) % R) * NB * PL;",
-         "      if (vst) {",
+         "      if constexpr (!vec) {",
+         "#pragma unroll",
+         "        for (int j = 0; j < RW; ++j)",
+         "          if (yo[j] >= 0) {",
+         "#pragma unroll",
+         "            for (int b = 0; b < NB; ++b)",
+         "#pragma unroll",
+         "              for (int k = 0; k < CE; ++k)",
+         "                if (xo[k] >= 0) xg_cp_async(slot + b * PL + (warp + NW * j) * PX + V - 1 + lane + 32 * k, "
+         "src[b] + zb + yo[j] + xo[k]);",
+         "          }",
+         "      } else if (vst) {",
          "#pragma unroll",
          "        for (int b = 0; b < NB; ++b)",
          "#pragma unroll",
@@ -1054,12 +1113,14 @@ def zstage_frame(kname: str, ptype: str, T: str, srcs: list, loads: list, outs: 
          "    }",
          "    xg_cp_async_commit();",
          "  };",
-         "#pragma unroll",
-         "  for (int q = 0; q < D + 2; ++q) stage(z0 - 1 + q);  // planes z0 - 1 .. z0 + D",
          "  const int tx_t = tid % NTX, ty_t = tid / NTX;",
          "  const int c0 = V + V * tx_t, x = x0 + V * tx_t;  // the thread's first cell: ring column, grid x",
+         *old,
+         "#pragma unroll",
+         "  for (int q = 0; q < D + 2; ++q) stage(z0 - 1 + q);  // planes z0 - 1 .. z0 + D",
          "  XG_ZSTAGE_WINDOW",
          "  for (int z = z0; z < z1; ++z) {",
+         "    old_planes(z + D);" if old else "",
          "    stage(z + D + 1);  // into the slot of plane z + D + 2 - R, read for the last time before the",
          "                       // previous plane's first barrier (R = D + 4) or its second (R = D + 3)",
          "    xg_cp_async_wait_group<D>();  // planes up to z + 1 have landed",
@@ -1126,7 +1187,11 @@ def zstage_frame(kname: str, ptype: str, T: str, srcs: list, loads: list, outs: 
             ind += "  "
         vals = ", ".join(f"o{o}[{j}]" for j in range(V))
         if acc:
-            K.append(f"{ind}{VT} a = *reinterpret_cast<const {VT}*>(&{dst}[gb]);")
+            if old:
+                K.append(f"{ind}const {VT} a = olds[(((z - z0) % (D + 1)) * {len(accs)} * {RY} + {accs.index(o) * RY} + i) "
+                         "* NT];")
+            else:
+                K.append(f"{ind}const {VT} a = *reinterpret_cast<const {VT}*>(&{dst}[gb]);")
             vals = ", ".join(f"a.{comp[j]} + (o{o}[{j}])" for j in range(V))
         K.append(f"{ind}*reinterpret_cast<{VT}*>(&{dst}[gb]) = make_{VT}({vals});")
         if guard:
@@ -1159,30 +1224,36 @@ def zstage_frame(kname: str, ptype: str, T: str, srcs: list, loads: list, outs: 
 
 
 def zstage_launch(kname: str, T: str, nb: int, ind: str, aligned: list, before: list, after: list,
-                  only_aligned: bool = False) -> list:
+                  only_aligned: bool = False, nacc: int = 0) -> list:
     """Host lines launching ``kname`` (a ``zstage_frame`` kernel) with parameters
     ``p`` on stream ``s`` when its shared memory fits; ``aligned``: the pointers
     (sources and destinations) that must be 16-byte aligned for 16-byte copies;
     ``before`` / ``after`` run around the launch, which ends with ``return 0``.
     Falls through otherwise (with ``only_aligned`` also where rows are unaligned)."""
-    g = zstage_geometry(T, nb)
+    g = zstage_geometry(T, nb, nacc)
     ty, tx = ZSTAGE_TILE
     al = " && ".join(f"((uintptr_t)({a}) & 15) == 0" for a in aligned) or "1"
+    # (vec, index type) of the instantiations; a kernel of unaligned rows has no old values to stage
+    kinds = [(v, it) for v in ((1,) if only_aligned else (1, 0)) for it in ("int", "int64_t")]
     L = ["{",
-         f"  const size_t smem = {g['smem']};",
-         "  static int avail32 = -1, avail64 = -1;",
-         "  const bool small = xg_small_index(p.Z, p.Y, p.X);",
-         f"  if (small && avail32 < 0) XG_TRY(xg_smem_optin({kname}<int>, &avail32));",
-         f"  if (!small && avail64 < 0) XG_TRY(xg_smem_optin({kname}<int64_t>, &avail64));",
-         "  int zlen = 0;",
-         "  int64_t nt = 0;",
-         f"  XG_TRY(xg_zstage_chunks(p.Z, p.Y, p.X, {ty}, {tx}, &zlen, &nt));",
          f"  const int vec = (p.X % {g['V']}) == 0 && {al};",
-         f"  if ({'vec && ' if only_aligned else ''}smem <= (size_t)(small ? avail32 : avail64) && nt <= 0x7fffffffLL) {{"]
+         f"  const size_t smem = vec ? {g['smem']} : {g['smem'] - g['acc']};",
+         "  static int avail[2][2] = {{-1, -1}, {-1, -1}};",
+         "  const bool small = xg_small_index(p.Z, p.Y, p.X);"]
+    for v, it in kinds:
+        cond = f"{'' if v else '!'}vec && {'' if it == 'int' else '!'}small"
+        L.append(f"  if ({cond} && avail[vec][small] < 0) "
+                 f"XG_TRY(xg_smem_optin({kname}<{it}, {'true' if v else 'false'}>, &avail[vec][small]));")
+    L += ["  int zlen = 0;",
+          "  int64_t nt = 0;",
+          f"  XG_TRY(xg_zstage_chunks(p.Z, p.Y, p.X, {ty}, {tx}, &zlen, &nt));",
+          f"  if ({'vec && ' if only_aligned else ''}smem <= (size_t)avail[vec][small] && nt <= 0x7fffffffLL) {{"]
     L += ["    " + b for b in before]
-    L += [f"    if (small) {kname}<int><<<(unsigned)nt, {ZSTAGE_THREADS}, smem, s>>>(p, zlen, vec);",
-          f"    else {kname}<int64_t><<<(unsigned)nt, {ZSTAGE_THREADS}, smem, s>>>(p, zlen, vec);",
-          "    XG_CUDA(cudaGetLastError());"]
+    for v, it in kinds:
+        cond = f"{'' if v else '!'}vec && {'' if it == 'int' else '!'}small"
+        L.append(f"    if ({cond}) {kname}<{it}, {'true' if v else 'false'}>"
+                 f"<<<(unsigned)nt, {ZSTAGE_THREADS}, smem, s>>>(p, zlen);")
+    L.append("    XG_CUDA(cudaGetLastError());")
     L += ["    " + a for a in after]
     L += ["    return 0;", "  }", "}"]
     return [ind + line for line in L]

@@ -760,10 +760,11 @@ static inline int xg_smem_optin(K* kernel, int* avail) {
 
 // Chunk length along z of a staged z-walk launch over a Z x Y x X grid cut into
 // (ty, tx) column blocks, one CTA per (block, chunk): the chunk count per column
-// minimises ceil(CTAs / SMs) * (planes per chunk + 1), the planes that the
-// busiest SM streams when every CTA costs its own planes plus its two halo
-// planes at half weight (neighbouring chunks read them too, often from L2).
-// Chunks hold at least 8 planes.  *nt receives the CTA count.
+// minimises the time of the busiest SM, (planes per chunk + 3 for the first planes) times
+// the time of a plane of its CTAs: 0.40 us each from three CTAs on, but 0.74 us for one
+// and 0.92 us for two, which wait for their copies (256 x 256 planes, FP32, two buffers).
+// 32, 64, 96, 256 planes: 13.1, 17.9, 22.9, 50.6 us; counting a lone CTA's planes like those
+// of three: 16.7, 29.0, 22.9, 50.2 us.  Chunks hold at least 8 planes.  *nt: the CTA count.
 static inline int xg_zstage_chunks(int64_t Z, int64_t Y, int64_t X, int ty, int tx, int* zlen, int64_t* nt) {
   int nsm = 0;
   XG_TRY(xg_sm_count(&nsm));
@@ -773,7 +774,7 @@ static inline int xg_zstage_chunks(int64_t Z, int64_t Y, int64_t X, int ty, int 
   int64_t best_len = Z, best_cost = -1;
   for (int64_t c = 1; c <= cmax; ++c) {
     const int64_t len = (Z + c - 1) / c, chunks = (Z + len - 1) / len;
-    const int64_t cost = ((ncb * chunks + nsm - 1) / nsm) * (len + 1);
+    const int64_t ctas = (ncb * chunks + nsm - 1) / nsm, cost = (len + 3) * (ctas == 1 ? 19 : ctas == 2 ? 23 : 10 * ctas);
     if (best_cost < 0 || cost < best_cost) {
       best_cost = cost;
       best_len = len;
