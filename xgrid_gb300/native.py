@@ -21,6 +21,9 @@ from .grid import Grid
 from .log import Logger
 from .types import Number, Structure, Void
 
+# argument types whose conversion a structure's constructor does as the field types' serialize()
+_PLAIN = {bool, int, float}
+
 
 class NativeKernel:
     def __init__(self, operator) -> None:
@@ -205,7 +208,7 @@ class NativeKernel:
         return ev
 
     def pack(self, values: list):
-        if self.plain_values:
+        if self.plain_values and _PLAIN.issuperset(map(type, values)):
             return self.args_type(*values[: len(self.module.value_args)])
         packed = self.args_type()
         for (name, t), v in zip(self.module.value_args, values):
