@@ -19,7 +19,10 @@ rows of 3-D grids) and walks a chunk of the slowest axis:
   where the CTA's next warp holds them).
 
 Boundary cells: one bit per cell (``xg_mask_bits``) tells the cells that the sweep leaves
-alone, and the group's boundary phases follow as launches over their cell lists.  The chunk
+alone, and the group's boundary phases follow as launches over their cell lists.  A row's mask
+words are loaded with the planes ahead, one word a lane, and handed round by shuffles (loaded by
+every lane where its cells are stored, they cost an L1 or L2 latency per row: 256^3 walls 51 us
+against 44; two bits per cell and the phases' constants stored by the sweep itself: 47).  The chunk
 length comes from the SM count, so that the strips fill whole rounds of the resident warps.
 Same arithmetic per cell as the other paths.
 """
@@ -30,7 +33,8 @@ from . import analysis
 WARPS = 4              # warps per CTA
 # (segments of 32 columns, rows, planes ahead, resident CTAs per SM asked of ptxas), by dimension
 # and loaded buffers; wide strips first.  Measured: 4096^2 transport 29 us (2 rows ahead; with 4:
-# 31, with 2 segments 39); 256^3 walls 51 us with 8 segments, 58 with 2 x 2; 203 x 245 x 307
+# 31, with 2 segments 39); 256^3 walls 51 us with 8 segments, 58 with 2 x 2 (before the mask
+# words were loaded ahead; 44 since); 203 x 245 x 307
 # diffusion 56 us (4 x 1: 64, 1 x 4: 66).
 SHAPE = {(2, 1): [(4, 1, 2, 6)], (2, 2): [(2, 1, 2, 6)], (3, 1): [(8, 1, 1, 4), (2, 2, 1, 6)], (3, 2): [(2, 2, 1, 4)]}
 FILL = 60  # a strip shape applies where the grid's columns fill at least this share (%) of its lanes
@@ -164,6 +168,14 @@ def _kernel(em, tag: str, j: int, pl, variant: int, shape: tuple) -> str:
                 out.append(f"          {sd}[r][{k}] = {who} && oka && ok_row(q + {x}) ? {v}_s[q + {x}] : ({t})0;")
             out.append("        }")
         return out + ["      }"]
+    K += ["  // mask words of the strip's rows, lane j holding those of columns 32 j: loaded with the planes ahead",
+          "  const int W = (X + 31) / 32, wx = x0 / 32 + lane;",
+          "  uint32_t wc[U][R], wn[U][R];",
+          "  auto words = [&](uint32_t (&w)[R], int a) {",
+          "#pragma unroll", "    for (int r = 0; r < R; ++r)",
+          "      w[r] = MASKED && a < ab && y0 + r < NY && lane < J && wx < W ? bits[((I)a * NY + y0 + r) * W + wx] : 0u;",
+          "  };",
+          "#pragma unroll", "  for (int u = 0; u < U; ++u) words(wc[u], aa + u);"]
     for b in bufs:
         v, np_ = em.bname(b), hi[b] - lo[b]
         K += ["#pragma unroll", f"  for (int k = 0; k < U + {np_}; ++k) {{"]
@@ -173,7 +185,7 @@ def _kernel(em, tag: str, j: int, pl, variant: int, shape: tuple) -> str:
             K += load_rim(b, f"h{v}[u]", f"s{v}[u]", "aa + u", "aa + u < ab") + ["  }"]
     K += ["#pragma unroll 1", "  for (int a = aa; a < ab; a += U) {",
           "    // the next planes and their rim",
-          "#pragma unroll", "    for (int u = 0; u < U; ++u) {"]
+          "#pragma unroll", "    for (int u = 0; u < U; ++u) {", "      words(wn[u], a + U + u);"]
     for b in bufs:
         v = em.bname(b)
         K += load_plane(b, f"n{v}[u]", f"a + U + u + ({hi[b]})", f"a + U + u + ({hi[b]}) <= ab")
@@ -217,7 +229,7 @@ def _kernel(em, tag: str, j: int, pl, variant: int, shape: tuple) -> str:
     val = gen.expr(s.stmt.value, env)
     K += ["          bool live = in[j];",
           "          if (MASKED) {  // bit set: the sweep leaves the cell alone",
-          f"            const uint32_t word = live ? bits[((I)(a + u) * NY + y0 + r) * ((X + 31) / 32) + (x0 >> 5) + j] : 0u;"]
+          "            const uint32_t word = __shfl_sync(FULL, wc[u][r], j);"]
     if s.implicit:
         b = (s.slot, s.level, s.read_version_of_target)
         K.append(f"            if (live && (word >> lane & 1u)) out[q + 32 * j] = c{em.bname(b)}[u + {-lo[b]}][r][j];")
@@ -235,7 +247,8 @@ def _kernel(em, tag: str, j: int, pl, variant: int, shape: tuple) -> str:
         if side[b]:
             K += ["#pragma unroll", "    for (int u = 0; u < U; ++u)", "#pragma unroll",
                   f"      for (int r = 0; r < R; ++r) {{ s{v}[u][r][0] = sn{v}[u][r][0]; s{v}[u][r][1] = sn{v}[u][r][1]; }}"]
-    K += ["  }", "}"]
+    K += ["#pragma unroll", "    for (int u = 0; u < U; ++u)", "#pragma unroll",
+          "      for (int r = 0; r < R; ++r) wc[u][r] = wn[u][r];", "  }", "}"]
     return "\n".join(K)
 
 
