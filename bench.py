@@ -941,13 +941,17 @@ def batch_section(count: int, steps: int, seq_steps: int) -> dict:
     out["e2e"] = {"value": cells * steps / e2e_s / 1e9, "unit": "GLUP/s", "h2d_bytes_per_step": 4 * cells,
                   "d2h_bytes_per_step": 4 * cells, "ms": e2e_s * 1e3,
                   "step": f"one call of {steps} steps from host arrays to host arrays"}
-    cpu = bounded_steps("convdiff", 0, 10.0, 50)
-    out["cpu_baseline"] = {"value": cpu["cells"] * cpu["steps"] / cpu["seconds"] / 1e9, "unit": "GLUP/s",
-                           "cores": cpu["cores"], "kind": cpu["kind"],
-                           "sample": f"reference C, one call per problem per step, {count} squares of the problems' "
-                                     f"cell counts ({cpu['cells']} cells), {cpu['steps']} steps "
-                                     f"({cpu['seconds']:.1f} s); timing only (the reference mis-indexes non-square "
-                                     f"grids), OpenMP on all host cores"}
+    from oracle import native
+    if any(os.path.exists(os.path.join(native.REF, "convdiff2d" + e)) for e in (".c", ".so")):
+        cpu = bounded_steps("convdiff", 0, 10.0, 50)
+        out["cpu_baseline"] = {"value": cpu["cells"] * cpu["steps"] / cpu["seconds"] / 1e9, "unit": "GLUP/s",
+                               "cores": cpu["cores"], "kind": cpu["kind"],
+                               "sample": f"reference C, one call per problem per step, {count} squares of the problems' "
+                                         f"cell counts ({cpu['cells']} cells), {cpu['steps']} steps "
+                                         f"({cpu['seconds']:.1f} s); timing only (the reference mis-indexes non-square "
+                                         f"grids), OpenMP on all host cores"}
+    else:
+        out["cpu_baseline"] = {"unavailable": "the reference's generated C of this program is not in the working tree"}
     out["config"] = (f"{count} problems, extents U[64,1024] per axis (seed 1), FP32, periodic, convection-diffusion "
                      f"5-point, {steps} steps in one CUDA graph of persistent launches")
     return out
