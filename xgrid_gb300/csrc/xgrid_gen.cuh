@@ -645,6 +645,32 @@ static inline double xg_boxes_cost(int64_t nb, int sms, int per_sm, int nt, int 
   return (t + 2500 * rounds) / th;
 }
 
+// The core rows, box width and depth (t0 to t1 iterations) of boxes on a Y x X grid with the
+// least cost per iteration; `most` CTAs of `nt` threads at most on an SM, `cell` bytes of
+// shared memory per box cell.
+struct xg_box_shape {
+  int cy, bx, th;
+};
+static inline void xg_boxes_search(int64_t Y, int64_t X, int sms, int most, int nt, size_t cell, int ops, int t0, int t1,
+                                   struct xg_box_shape* out) {
+  double best = -1;
+  for (int t = t0; t <= t1; ++t)
+    for (int w : {32, 64, 96, 128}) {
+      const int cx = w - 2 * t;
+      for (int r = 4; cx >= 8 && r <= 64; ++r) {
+        const size_t smem = (size_t)(r + 2 * t) * w * cell;
+        const int fit = (int)((228 * 1024) / (smem + 1024)), per_sm = fit < most ? fit : most;
+        if (per_sm < 1) continue;
+        const int64_t nb = ((Y + r - 1) / r) * ((X + cx - 1) / cx);
+        const double cost = xg_boxes_cost(nb, sms, per_sm, nt, ops, r, w, t);
+        if (best < 0 || cost < best) {
+          best = cost;
+          *out = {r, w, t};
+        }
+      }
+    }
+}
+
 // ---------------------------------------------------------------------------
 // Power-of-two storage scales of 16-bit fields.  For a field whose largest
 // magnitude is m, xg_scale_exp(m, A) = A - floor(log2 m) (clamped to the normal

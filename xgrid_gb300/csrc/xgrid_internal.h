@@ -1,5 +1,6 @@
 // Runtime hooks used only by generated kernel modules (not part of the public C ABI).
 #pragma once
+#include "xgrid_gb300.h"
 
 #ifdef __cplusplus
 extern "C" {
@@ -9,6 +10,14 @@ extern "C" {
  * device memory for boundary-mask tables and reports an error instead.  The
  * no-alloc entry points of generated modules set it around their call. */
 void xg_internal_noalloc_scope(int on);
+
+/* 0 while a call on `stream` may not build boundary-mask tables: inside the scope
+ * above, and while the stream is being captured. */
+int xg_internal_may_build(void* stream);
+
+/* 1 when the box tables of (core, halo) and of every mask value listed are built. */
+int xg_internal_boxes_built(const xg_mask* mask, const int32_t* core, const int32_t* halo, int nvalues,
+                            const int32_t* values);
 
 #ifdef __cplusplus
 }

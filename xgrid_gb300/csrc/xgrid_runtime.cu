@@ -257,6 +257,24 @@ const char* xg_last_error(void) { return g_error.c_str(); }
 
 void xg_internal_noalloc_scope(int on) { g_noalloc_scope = on; }
 
+int xg_internal_may_build(void* stream) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  return !g_noalloc_scope && (cudaStreamIsCapturing(static_cast<cudaStream_t>(stream), &st) != cudaSuccess ||
+                              st == cudaStreamCaptureStatusNone);
+}
+
+int xg_internal_boxes_built(const xg_mask* m, const int32_t* core, const int32_t* halo, int nvalues,
+                            const int32_t* values) {
+  BoxKey key;
+  std::copy(core, core + 3, key.core);
+  std::copy(halo, halo + 3, key.halo);
+  const auto it = m->boxes.find(key);
+  if (it == m->boxes.end()) return 0;
+  for (int i = 0; i < nvalues; ++i)
+    if (!it->second.csr.count(values[i])) return 0;
+  return 1;
+}
+
 void xg_set_error(const char* message) { g_error = message ? message : ""; }
 
 int xg_runtime_version(void) { return 1; }

@@ -40,6 +40,7 @@ from . import analysis
 THREADS = 512
 DEEPEST = 6  # iterations of a launch that the depth rule may take (8: its boxes fail the check on small grids)
 SITE = 57  # profiling site of the launch within its group
+BOX_WIDTHS = (32, 64, 96, 128)  # as in xg_boxes_search
 MIN_BLOCKS = 2  # resident CTAs per SM asked of ptxas (4 of 256 threads: 4 to 10 % slower from 513^2 on)
 
 
@@ -88,23 +89,26 @@ def plan(em) -> dict | None:
     return {"slot": slot, "level": level, "main_offs": main_offs, "phases": phases}
 
 
-def fp64_ops(em, sweep) -> str:
-    """Host expression of the FP64 operations per cell of a sweep: products and quotients
-    by launch constants cost what their parameter says (none for powers of two)."""
+def fp64_ops(em, sweep) -> tuple[str, int, int]:
+    """FP64 operations per cell of a sweep: host expression, least and largest value.
+    Products and quotients by launch constants cost what their parameter says (none for
+    powers of two), so the count depends on the scalars of the call."""
     from . import ir
     from .codegen import has_stencil
-    n, terms = 0, []
+    n, most, terms = 0, 0, []
     for e in ir.walk(sweep.stmt.value):
         if not isinstance(e, ir.Binary) or not has_stencil(e) or em.gen.ctype(e) != "double":
             continue
         if id(e) in em.div_map:
             k = f"h->{em.div_map[id(e)].name}"
             terms.append(f"({k}.rz.p2 ? 0 : ({k}.two ? 2 : 4))")
+            most += 4
         elif id(e) in em.mul_map:
             terms.append(f"(h->{em.mul_map[id(e)][0].name}.p2 ? 0 : 1)")
+            most += 1
         elif not e.operator.is_compare() and not e.operator.is_logic():
             n += 1
-    return " + ".join([str(n)] + terms)
+    return " + ".join([str(n)] + terms), n, n + most
 
 
 def emit(em, th: int) -> None:
@@ -225,7 +229,7 @@ def emit(em, th: int) -> None:
     def arr(name, typ, xs):
         return [f"  static const {typ} {name}[] = {{{', '.join(str(v) for v in xs) if xs else '0'}}};"]
     site = gid * 64 + SITE
-    bxs = (32, 64, 96, 128)
+    bxs = BOX_WIDTHS
     L = [f"static int xgl_{n}_{gid}_tloop(xg_grid* G, const struct xgh_{n}_{gid}* h, int64_t K, cudaStream_t s) {{",
          f"  if (!xg_tloop_{n} || G[{slot}].ndim != 2) return 0;"]
     L += em.check_levels(sweeps)
@@ -244,50 +248,53 @@ def emit(em, th: int) -> None:
     L += arr("mo", "int32_t", [v for t in mo for v in t]) + arr("vals", "int32_t", vals)
     L += arr("nof", "int32_t", nof) + arr("offs", "int32_t", offs)
     auto = gen.cfg.loop_auto
+    ops, least, most = fp64_ops(em, sweeps[0])
+    mask = f"G[{slot}].mask"
+    tables = [f"XG_TRY(xg_mask_boxes({mask}, core, halo, 0, &p.bzero, NULL, NULL, &nb));"]
+    tables += [f"XG_TRY(xg_mask_boxes({mask}, core, halo, {v}, NULL, &p.bo{j}, &p.bl{j}, &nb));"
+               for j, v, _ in pl["phases"]]
     L += ["  // iterations per launch, core rows and box width with the least time per iteration" +
           ("; at the\n  // configured depth where the mask does not allow the one that came out" if auto else ""),
-          f"  const int ops = {fp64_ops(em, sweeps[0])};  // FP64 operations per cell of the main sweep",
+          f"  const int ops = {ops};  // FP64 operations per cell of the main sweep",
+          f"  constexpr int OPS0 = {least}, NO = {most - least + 1};  // its values over all scalars",
           f"  constexpr int TH = {th};  // the configured depth" + (f"; the rule takes 2 to {DEEPEST}" if auto else ""),
           f"  constexpr int NC = {2 if auto else 1}, lo_th[] = {{{'2, TH' if auto else 'TH'}}}, "
           f"hi_th[] = {{{f'{DEEPEST}, TH' if auto else 'TH'}}};",
-          "  struct shape { int cy, bx, th; };",
           "  static thread_local int64_t key_y = -1, key_x = -1;",
-          "  static thread_local int key_ops = -1;",
-          "  static thread_local struct shape kept[NC];",
-          "  if (key_y != p.Y || key_x != p.X || key_ops != ops) {",
-          "    int sms = 0;",
-          "    XG_TRY(xg_sm_count(&sms));",
-          "    for (int c = 0; c < NC; ++c) {",
-          "      double best = -1;",
-          "      for (int t = lo_th[c]; t <= hi_th[c]; ++t)",
-          f"        for (int w : {{{', '.join(str(v) for v in bxs)}}}) {{",
-          "          const int cx = w - 2 * t;",
-          "          for (int r = 4; cx >= 8 && r <= 64; ++r) {",
-          f"            const size_t smem = (size_t)(r + 2 * t) * w * (2 * sizeof({T}) + sizeof(int32_t));",
-          f"            const int fit = (int)((228 * 1024) / (smem + 1024)), per_sm = fit < {MIN_BLOCKS} ? fit : {MIN_BLOCKS};",
-          "            if (per_sm < 1) continue;",
-          "            const int64_t nb = ((p.Y + r - 1) / r) * ((p.X + cx - 1) / cx);",
-          f"            const double cost = xg_boxes_cost(nb, sms, per_sm, {THREADS}, ops, r, w, t);",
-          "            if (best < 0 || cost < best) { best = cost; kept[c] = {r, w, t}; }",
-          "          }",
-          "        }",
-          "    }",
-          "    key_y = p.Y; key_x = p.X; key_ops = ops;",
+          "  static thread_local struct xg_box_shape kept[NO][NC];  // th 0: not worked out yet",
+          "  if (key_y != p.Y || key_x != p.X) {",
+          "    memset(kept, 0, sizeof kept);",
+          "    key_y = p.Y; key_x = p.X;",
           "  }",
+          "  int sms = 0;",
+          "  XG_TRY(xg_sm_count(&sms));",
           "  int cy = 0, bx = 0, D = 0, ok = 0;",
           "  int32_t core[3] = {1, 1, 1}, halo[3] = {0, 0, 0};",
           "  const int32_t shrink[3] = {0, 1, 1};",
-          "  for (int c = 0; c < NC && !ok; ++c) {",
-          "    cy = kept[c].cy; bx = kept[c].bx; D = kept[c].th;",
+          "  // class c's shape for o operations, and whether the mask allows it",
+          "  auto take = [&](int o, int c, int* allowed) {",
+          "    struct xg_box_shape* k = &kept[o - OPS0][c];",
+          f"    if (k->th == 0) xg_boxes_search(p.Y, p.X, sms, {MIN_BLOCKS}, {THREADS}, 2 * sizeof({T}) + sizeof(int32_t), o, "
+          "lo_th[c], hi_th[c], k);",
+          "    cy = k->cy; bx = k->bx; D = k->th;",
           "    core[1] = cy; core[2] = bx - 2 * D; halo[1] = halo[2] = D;",
-          f"    XG_TRY(xg_mask_box_check(G[{slot}].mask, core, halo, shrink, D, {len(mo)}, mo, {len(vals)}, vals, nof, "
-          "offs, &ok));",
-          "  }",
+          f"    return xg_mask_box_check({mask}, core, halo, shrink, D, {len(mo)}, mo, {len(vals)}, vals, nof, offs, allowed);",
+          "  };",
+          "  int c = 0;",
+          "  for (; c < NC && !ok; ++c) XG_TRY(take(ops, c, &ok));",
           "  if (!ok) return 0;",
-          "  int64_t nb = 0;",
-          f"  XG_TRY(xg_mask_boxes(G[{slot}].mask, core, halo, 0, &p.bzero, NULL, NULL, &nb));"]
-    for j, v, _ in pl["phases"]:
-        L.append(f"  XG_TRY(xg_mask_boxes(G[{slot}].mask, core, halo, {v}, NULL, &p.bo{j}, &p.bl{j}, &nb));")
+          "  // a call that may not build tables takes whichever shape an earlier call built them for, with",
+          "  // whatever scalars: every shape gives the same bits",
+          f"  if (!xg_internal_may_build(s) && !xg_internal_boxes_built({mask}, core, halo, {len(vals)}, vals)) {{",
+          "    int built = 0;",
+          "    for (int i = 0; i < NO * NC && !built; ++i) {",
+          "      XG_TRY(take(OPS0 + i / NC, i % NC, &ok));",
+          f"      built = ok && xg_internal_boxes_built({mask}, core, halo, {len(vals)}, vals);",
+          "    }",
+          "    if (!built) XG_TRY(take(ops, c - 1, &ok));",
+          "  }",
+          "  int64_t nb = 0;"]
+    L += ["  " + x for x in tables]
     L += ["  // (the tables above exist from here on, also for calls of one iteration: a later call of",
           "  //  several may come from an entry that may not build them)",
           "  if (K < 2 || nb > 0x7fffffffLL) return 0;",
