@@ -352,6 +352,26 @@ static inline int xg_sm_count(int* sms) {
   return 0;
 }
 
+// How many parts, lo to hi, to cut `len` planes (rows) into, when every part is `per` units of
+// work on `slots` places: the least cost(rounds, planes per part), the smallest such count.
+// cost must grow with both.  Launch rules run at every call that is one launch, so the search
+// visits one count per number of rounds, its largest, instead of every count (strips of a
+// 65536 x 128 FP32 grid: 2 counts instead of 4096, 36.5 -> 14.4 us a call).
+template <typename F>
+static inline int64_t xg_best_parts(int64_t len, int64_t per, int64_t slots, int64_t lo, int64_t hi, F cost) {
+  int64_t count = lo, best = -1;
+  for (int64_t n = lo, last; n <= hi; n = last + 1) {
+    const int64_t rounds = (n * per + slots - 1) / slots;
+    last = rounds * slots / per < hi ? rounds * slots / per : hi;
+    const int64_t part = (len + last - 1) / last, c = cost(rounds, part);
+    if (best < 0 || c < best) {
+      best = c;
+      count = (len + part - 1) / part > n ? (len + part - 1) / part : n;
+    }
+  }
+  return count;
+}
+
 // The tiling of a launch: `cfg` when it was set for the group, else the default's columns
 // and threads, and a tile count along the slowest axis (a negative extent) that levels the
 // work where the default's does not.
@@ -364,6 +384,14 @@ static inline int xg_sm_count(int* sms) {
 // The default stays when it costs at most a tenth more (on 2-D grids the loops take its
 // 64 rows in whole passes, which a memory-bound sweep feels: 229 against 250 us for the
 // 4097^2 residual launch with 216 rows).
+static inline int64_t xg_tile_parts(int64_t len, int64_t per, int64_t slots, int64_t n0, int flat) {
+  const int64_t n1 = flat ? n0 : 1, nmax = len / (flat ? 4 : 8), hi = nmax < n1 + 256 ? nmax : n1 + 256;
+  if (hi < n1) return n0;
+  auto cost = [](int64_t rounds, int64_t part) { return rounds * (part + 2); };
+  const int64_t n = xg_best_parts(len, per, slots, n1, hi, cost);
+  auto of = [&](int64_t k) { return cost((k * per + slots - 1) / slots, (len + k - 1) / k); };
+  return 10 * of(n0) <= 11 * of(n) || n > 65535 ? n0 : n;
+}
 static inline const int32_t* xg_tiling_for(const int32_t* cfg, int set, const xg_grid* g, int blocks, int32_t* buf) {
   if (set || g->ndim < 2) return cfg;
   int sms = 0;
@@ -372,21 +400,11 @@ static inline const int32_t* xg_tiling_for(const int32_t* cfg, int set, const xg
   const int flat = g->ndim == 2;
   const int64_t len = flat ? e.y : e.z;
   const int64_t per = xg_tiles_along(e.x, cfg[2]) * (flat ? 1 : xg_tiles_along(e.y, cfg[1]));
-  const int64_t slots = flat ? sms : (int64_t)sms * blocks;
   const int64_t n0 = xg_tiles_along(len, cfg[flat ? 1 : 0]);
-  const int64_t n1 = flat ? n0 : 1, nmax = len / (flat ? 4 : 8);
-  int64_t best = -1, count = n0;
-  auto cost = [&](int64_t n) { return ((n * per + slots - 1) / slots) * ((len + n - 1) / n + 2); };
-  for (int64_t n = n1; n <= nmax && n <= n1 + 256; ++n) {
-    const int64_t c = cost(n);
-    if (best < 0 || c < best) {
-      best = c;
-      count = n;
-    }
-  }
-  if (best < 0 || 10 * cost(n0) <= 11 * best || count > 65535) return cfg;
+  const int64_t n = xg_tile_parts(len, per, flat ? sms : (int64_t)sms * blocks, n0, flat);
+  if (n == n0) return cfg;
   memcpy(buf, cfg, 6 * sizeof(int32_t));
-  buf[flat ? 1 : 0] = -(int32_t)count;
+  buf[flat ? 1 : 0] = -(int32_t)n;
   return buf;
 }
 
@@ -791,24 +809,20 @@ static inline int xg_smem_optin(K* kernel, int* avail) {
 // and 0.92 us for two, which wait for their copies (256 x 256 planes, FP32, two buffers).
 // 32, 64, 96, 256 planes: 13.1, 17.9, 22.9, 50.6 us; counting a lone CTA's planes like those
 // of three: 16.7, 29.0, 22.9, 50.2 us.  Chunks hold at least 8 planes.  *nt: the CTA count.
-static inline int xg_zstage_chunks(int64_t Z, int64_t Y, int64_t X, int ty, int tx, int* zlen, int64_t* nt) {
-  int nsm = 0;
-  XG_TRY(xg_sm_count(&nsm));
-  const int64_t ncb = ((X + tx - 1) / tx) * ((Y + ty - 1) / ty);
+static inline int64_t xg_zstage_length(int64_t Z, int64_t ncb, int sms) {
   int64_t cmax = Z / 8 > 1 ? Z / 8 : 1;
   if (cmax > 4096) cmax = 4096;
-  int64_t best_len = Z, best_cost = -1;
-  for (int64_t c = 1; c <= cmax; ++c) {
-    const int64_t len = (Z + c - 1) / c, chunks = (Z + len - 1) / len;
-    const int64_t ctas = (ncb * chunks + nsm - 1) / nsm, cost = (len + 3) * (ctas == 1 ? 19 : ctas == 2 ? 23 : 10 * ctas);
-    if (best_cost < 0 || cost < best_cost) {
-      best_cost = cost;
-      best_len = len;
-    }
-  }
-  if (best_len > 0x7fffffffLL) XG_FAIL("staged z-walk: chunk of %lld planes", (long long)best_len);
-  *zlen = (int)best_len;
-  *nt = ncb * ((Z + best_len - 1) / best_len);
+  const int64_t n = xg_best_parts(Z, ncb, sms, 1, cmax, [](int64_t ctas, int64_t len) {
+    return (len + 3) * (ctas == 1 ? 19 : ctas == 2 ? 23 : 10 * ctas);
+  });
+  return (Z + n - 1) / n;
+}
+static inline int xg_zstage_chunks(int64_t Z, int64_t Y, int64_t X, int ty, int tx, int* zlen, int64_t* nt) {
+  int sms = 0;
+  XG_TRY(xg_sm_count(&sms));
+  const int64_t ncb = ((X + tx - 1) / tx) * ((Y + ty - 1) / ty), len = xg_zstage_length(Z, ncb, sms);
+  *zlen = (int)len;
+  *nt = ncb * ((Z + len - 1) / len);
   return 0;
 }
 
@@ -817,20 +831,19 @@ static inline int xg_zstage_chunks(int64_t Z, int64_t Y, int64_t X, int ty, int 
 // the slowest axis that minimises ceil(warps / resident warps) * (planes per chunk + 3),
 // three planes standing for a chunk's first loads; chunks hold at least 8 planes.  *nw
 // receives the warp count.
+static inline int64_t xg_strip_length(int64_t A, int64_t strips, int64_t slots) {
+  int64_t cmax = A / 8 > 1 ? A / 8 : 1;
+  if (cmax > 4096) cmax = 4096;
+  const int64_t n = xg_best_parts(A, strips, slots, 1, cmax,
+                                  [](int64_t rounds, int64_t len) { return rounds * (len + 3); });
+  return (A + n - 1) / n;
+}
 static inline int xg_strip_chunks(int64_t A, int64_t NY, int64_t X, int w, int r, int warps_per_sm, int* alen,
                                   int64_t* nsx, int64_t* nsy, int64_t* nw) {
   int sms = 0;
   XG_TRY(xg_sm_count(&sms));
-  const int64_t nx = (X + w - 1) / w, ny = (NY + r - 1) / r, slots = (int64_t)sms * warps_per_sm;
-  int64_t best = -1, len = A;
-  for (int64_t c = 1; c <= (A / 8 > 1 ? A / 8 : 1) && c <= 4096; ++c) {
-    const int64_t l = (A + c - 1) / c, chunks = (A + l - 1) / l;
-    const int64_t cost = ((nx * ny * chunks + slots - 1) / slots) * (l + 3);
-    if (best < 0 || cost < best) {
-      best = cost;
-      len = l;
-    }
-  }
+  const int64_t nx = (X + w - 1) / w, ny = (NY + r - 1) / r;
+  const int64_t len = xg_strip_length(A, nx * ny, (int64_t)sms * warps_per_sm);
   *alen = (int)len;
   *nsx = nx;
   *nsy = ny;

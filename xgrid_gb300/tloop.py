@@ -260,11 +260,16 @@ def emit(em, th: int) -> None:
           f"  constexpr int TH = {th};  // the configured depth" + (f"; the rule takes 2 to {DEEPEST}" if auto else ""),
           f"  constexpr int NC = {2 if auto else 1}, lo_th[] = {{{'2, TH' if auto else 'TH'}}}, "
           f"hi_th[] = {{{f'{DEEPEST}, TH' if auto else 'TH'}}};",
-          "  static thread_local int64_t key_y = -1, key_x = -1;",
-          "  static thread_local struct xg_box_shape kept[NO][NC];  // th 0: not worked out yet",
-          "  if (key_y != p.Y || key_x != p.X) {",
-          "    memset(kept, 0, sizeof kept);",
-          "    key_y = p.Y; key_x = p.X;",
+          "  // shapes of the last grid sizes (th 0: not worked out yet; the search takes longer than a call",
+          "  // of one launch): by operation count and class",
+          "  static thread_local struct { int64_t y, x; struct xg_box_shape k[NO][NC]; } sizes[8];",
+          "  static thread_local unsigned turn = 0;",
+          "  auto* kept = &sizes[0];",
+          "  for (auto& e : sizes) if (e.y == p.Y && e.x == p.X) kept = &e;",
+          "  if (kept->y != p.Y || kept->x != p.X) {",
+          "    kept = &sizes[turn++ % 8];",
+          "    memset(kept, 0, sizeof *kept);",
+          "    kept->y = p.Y; kept->x = p.X;",
           "  }",
           "  int sms = 0;",
           "  XG_TRY(xg_sm_count(&sms));",
@@ -273,7 +278,7 @@ def emit(em, th: int) -> None:
           "  const int32_t shrink[3] = {0, 1, 1};",
           "  // class c's shape for o operations, and whether the mask allows it",
           "  auto take = [&](int o, int c, int* allowed) {",
-          "    struct xg_box_shape* k = &kept[o - OPS0][c];",
+          "    struct xg_box_shape* k = &kept->k[o - OPS0][c];",
           f"    if (k->th == 0) xg_boxes_search(p.Y, p.X, sms, {MIN_BLOCKS}, {THREADS}, 2 * sizeof({T}) + sizeof(int32_t), o, "
           "lo_th[c], hi_th[c], k);",
           "    cy = k->cy; bx = k->bx; D = k->th;",
