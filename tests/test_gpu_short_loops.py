@@ -54,3 +54,20 @@ def test_boxes_are_no_deeper_than_the_loop(cacheroot, precision, n, iters, depth
             assert len(_depths(p)) == 1 and _depths(p) <= depths
         out.append(p.read(0).tobytes())
     assert out[0] == out[1]
+
+
+@pytest.mark.parametrize("n,iters,direct", [(33, 1, False), (65, 3, False), (257, 2, False), (257, 3, False),
+                                            (1025, 3, True), (1500, 2, True)])
+def test_short_launches_replay_their_graph(cacheroot, n, iters, direct):
+    """A short launch is cheaper as a graph replay, which issues no launch of its own; a long
+    one is launched directly from the third call on."""
+    xgrid.init(precision="double", cacheroot=cacheroot, opt_level=3)
+    k = Operator(relax, "kernel", "relax")
+    p, f = _grids(n)
+    for _ in range(8):  # every rotation of the levels eager, then captured
+        k(p, f, iters)
+    lib = runtime.load()
+    before = lib.xg_prof_launches()
+    for _ in range(4):
+        k(p, f, iters)
+    assert lib.xg_prof_launches() - before == (4 if direct else 0)

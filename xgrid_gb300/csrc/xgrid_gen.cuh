@@ -652,6 +652,7 @@ __device__ __forceinline__ void xg_tile_done(unsigned* flags, int64_t t, unsigne
 // cavity steps (us, against 3 iterations in boxes that minimise cells per CTA slot):
 // 129^2 144 -> 109, 257^2 165 -> 151, 513^2 270 -> 269, 700^2 739 -> 682, 1025^2 722 -> 698,
 // 1200^2 1786 -> 1703, 1500^2 2564 -> 2472.
+enum { XG_CYCLES_PER_US = 2070 };  // at the maximum SM clock
 static inline double xg_boxes_cost(int64_t nb, int sms, int per_sm, int nt, int ops, int r, int w, int th) {
   const int64_t most = (nb + sms - 1) / sms, rounds = (most + per_sm - 1) / per_sm;
   double t = 6000;

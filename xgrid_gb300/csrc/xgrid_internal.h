@@ -19,6 +19,11 @@ int xg_internal_may_build(void* stream);
 int xg_internal_boxes_built(const xg_mask* mask, const int32_t* core, const int32_t* halo, int nvalues,
                             const int32_t* values);
 
+/* Called by an entry whose one launch is short (about 12 us on the GPU at most): xg_call
+ * then replays its graph, the cheaper call on the host, instead of launching directly,
+ * which leaves a shorter gap on the GPU. */
+void xg_internal_short_launch(void);
+
 #ifdef __cplusplus
 }
 #endif

@@ -34,6 +34,8 @@ thread_local std::string g_error;
 std::atomic<uint64_t> g_mask_versions{0};
 // set while a no-alloc entry point runs: building a missing table is an error
 thread_local int g_noalloc_scope = 0;
+// set by an entry that runs: its one launch is shorter than a call takes on the host
+thread_local bool g_short_launch = false;
 
 int fail(const std::string& msg) {
   g_error = msg;
@@ -213,7 +215,8 @@ inline int64_t inner_distance(int64_t x, int64_t i, int32_t c, int32_t h, int64_
 struct GraphEntry {
   std::vector<uint8_t> key;
   bool captured = false;
-  bool direct = false;  // one node: a plain launch is cheaper than a graph's (512^2 heat: 8 us against 12 on the GPU)
+  bool direct = false;  // one node: a plain launch is cheaper than a graph's on the GPU (1024^2 FP32 sweep: 8.3 us against
+                        // 9.3), unless the entry says that it is short
   cudaGraphExec_t exec = nullptr;
   std::vector<std::array<void*, XG_MAX_LEVELS + 1>> post;  // level[] + scratch per grid
   std::vector<uint8_t> ret;
@@ -256,6 +259,8 @@ int xg_graph_clear(xg_entry_fn fn);
 const char* xg_last_error(void) { return g_error.c_str(); }
 
 void xg_internal_noalloc_scope(int on) { g_noalloc_scope = on; }
+
+void xg_internal_short_launch(void) { g_short_launch = true; }
 
 int xg_internal_may_build(void* stream) {
   cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
@@ -704,6 +709,7 @@ int xg_call(xg_entry_fn fn, xg_grid* grids, int ngrids, const void* args, size_t
   }
   if (!e.captured) {
     XG_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
+    g_short_launch = false;
     int rc = fn(grids, ngrids, args, nargs, ret, nret, stream);
     cudaGraph_t graph = nullptr;
     cudaError_t ce = cudaStreamEndCapture(s, &graph);
@@ -718,7 +724,7 @@ int xg_call(xg_entry_fn fn, xg_grid* grids, int ngrids, const void* args, size_t
     cudaGraphDestroy(graph);
     if (ie != cudaSuccess) return cuda_fail(ie, "cudaGraphInstantiate");
     e.captured = true;
-    e.direct = nodes == 1;
+    e.direct = nodes == 1 && !g_short_launch;
     e.post.resize(ngrids);
     for (int i = 0; i < ngrids; ++i) {
       std::copy(grids[i].level, grids[i].level + XG_MAX_LEVELS, e.post[i].begin());

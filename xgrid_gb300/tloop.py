@@ -306,6 +306,12 @@ def emit(em, th: int) -> None:
     L += ["  " + x for x in tables]
     L += ["  // (the tables above exist from here on, also for calls of one iteration: a later call of",
           "  //  several may come from an entry that may not build them)",
+          "  {  // a graph costs less on the host than the launch of these boxes, and small ones are bound by the host:",
+          "     // 11.1 against 13.0 us a call of 3 iterations at 257^2; at 700^2 the GPU's 18.5 against 16.6 of 2 iterations",
+          f"    const size_t smem = (size_t)(cy + 2 * D) * bx * (2 * sizeof({T}) + sizeof(int32_t));",
+          f"    const int fit = (int)((228 * 1024) / (smem + 1024)), per_sm = fit < {MIN_BLOCKS} ? fit : {MIN_BLOCKS};",
+          f"    if (xg_boxes_cost(nb, sms, per_sm, {THREADS}, ops, cy, bx, D) * D < 12 * XG_CYCLES_PER_US) xg_internal_short_launch();",
+          "  }",
           "  if (K < 2 || nb > 0x7fffffffLL) return 0;",
           f"  p.m = xg_mask_device(G[{slot}].mask);",
           "  p.cy = cy; p.cx = bx - 2 * D; p.th = D;",
