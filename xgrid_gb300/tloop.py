@@ -291,17 +291,17 @@ def emit(em, th: int) -> None:
           f"  int c = {'K == 2 ? 2 : K <= TH ? 1 : 0' if auto else '0'};",
           "  XG_TRY(take(ops, c, &ok));",
           *(["  if (!ok && c != 1) XG_TRY(take(ops, c = 1, &ok));"] if auto else []),
-          "  if (!ok) return 0;",
           "  // a call that may not build tables takes whichever shape an earlier call built them for, with",
-          "  // whatever scalars: every shape gives the same bits",
-          f"  if (!xg_internal_may_build(s) && !xg_internal_boxes_built({mask}, core, halo, {len(vals)}, vals)) {{",
-          "    int built = 0;",
-          "    for (int i = 0; i < NO * NC && !built; ++i) {",
+          "  // whatever scalars and iterations: every shape gives the same bits.  Where there is none (the mask",
+          "  // did not allow the earlier call's shape), one launch per iteration, as the earlier call ran",
+          f"  if (!xg_internal_may_build(s) && !(ok && xg_internal_boxes_built({mask}, core, halo, {len(vals)}, vals))) {{",
+          "    ok = 0;",
+          "    for (int i = 0; i < NO * NC && !ok; ++i) {",
           "      XG_TRY(take(OPS0 + i / NC, i % NC, &ok));",
-          f"      built = ok && xg_internal_boxes_built({mask}, core, halo, {len(vals)}, vals);",
+          f"      ok = ok && xg_internal_boxes_built({mask}, core, halo, {len(vals)}, vals);",
           "    }",
-          "    if (!built) XG_TRY(take(ops, c, &ok));",
           "  }",
+          "  if (!ok) return 0;",
           "  int64_t nb = 0;"]
     L += ["  " + x for x in tables]
     L += ["  // (the tables above exist from here on, also for calls of one iteration: a later call of",
