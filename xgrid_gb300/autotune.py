@@ -224,7 +224,9 @@ def group_candidates(ndim: int) -> list:
 def tune(op, *args, calls: int = 2) -> dict:
     """Pick the tile shape of every launch group of kernel ``op`` for these
     arguments (one group at a time, the others at their current tiling) and
-    apply it; returns {group: tiling}."""
+    apply it; returns {group: tiling}.  A group that is fastest untuned (strips, tile
+    counts by the grid's extents) stays untuned, and its default tiling is returned:
+    4096^2 FP32 transport takes 28.7 us a call on strips and 45 on the best tiles."""
     from .config import get_config
     from .native import NativeKernel
     cfg = get_config()
@@ -236,10 +238,9 @@ def tune(op, *args, calls: int = 2) -> dict:
     hit = _load(cfg.cacheroot).get(key)
     groups = list(range(nk.module.groups))
     if hit is not None:
-        chosen = {int(g): tuple(t) for g, t in hit.items()}
-        for g, t in chosen.items():
-            nk.set_tiling(g, t)
-        return chosen
+        for g, t in hit.items():
+            nk.set_tiling(int(g), t)
+        return {int(g): nk._tiling_key(int(g)) for g in hit}
     ndim = max(len(g.shape) for g in grids)
     t = device.torch()
     sms = t.cuda.get_device_properties(t.cuda.current_device()).multi_processor_count
@@ -255,9 +256,9 @@ def tune(op, *args, calls: int = 2) -> dict:
             op(*args)
     try:
         for g in groups:
-            base = nk._tiling_key(g)
+            base = [nk._tiling_key(g)] if nk.tiling_is_set(g) else []
             results = []
-            for c in [base] + [c for c in cands if c != base]:
+            for c in [None] + base + [c for c in cands if c not in base]:
                 nk.set_tiling(g, c)
                 try:
                     results.append((_time(run), c))
@@ -265,9 +266,9 @@ def tune(op, *args, calls: int = 2) -> dict:
                     logger.info(f"group {g} tiling {c} skipped: {err}")
             ms, best = min(results, key=lambda r: r[0])
             nk.set_tiling(g, best)
-            chosen[g] = tuple(best)
+            chosen[g] = best
     finally:
         snap.restore()
-    _store(cfg.cacheroot, key, {str(g): list(t) for g, t in chosen.items()})
+    _store(cfg.cacheroot, key, {str(g): t and list(t) for g, t in chosen.items()})
     logger.info(f"{nk.module.name}: tilings {chosen}")
-    return chosen
+    return {g: nk._tiling_key(g) for g in chosen}

@@ -586,6 +586,10 @@ class CudaGenerator:
             src.append("  {" + ", ".join(str(v) for v in self.group_tiling.get(gi, DEFAULT_TILING[2])) + "},")
         src.append("};")
         src.append(f"static uint8_t xg_tiling_set_{name}[{max(self.group_counter[0], 1)}];  // set by xg_config: used as is")
+        src.append(f"static const int32_t xg_tiling_default_{name}[{max(self.group_counter[0], 1)}][6] = {{")
+        for gi in range(max(self.group_counter[0], 1)):
+            src.append("  {" + ", ".join(str(v) for v in self.group_tiling.get(gi, DEFAULT_TILING[2])) + "},")
+        src.append("};")
         batch_host = None
         from . import batch as batch_mod
         if (not device_only and batch_mod.qualifies(self) and len(self.group_emitters) == 1
@@ -601,8 +605,9 @@ class CudaGenerator:
         src.append(f'extern "C" int xg_config_{name}(int group, const int32_t* cfg, int fuse) {{')
         src.append(f"  if (fuse >= 0) xg_fuse_{name} = fuse;")
         src.append(f"  if (group < 0 || group >= {self.group_counter[0]} || !cfg) return 0;")
-        src.append(f"  for (int i = 0; i < 6; ++i) xg_tiling_{name}[group][i] = cfg[i];")
-        src.append(f"  xg_tiling_set_{name}[group] = 1;")
+        src.append("  const int set = cfg[0] != 0;  // zeros: back to the launch rules")
+        src.append(f"  for (int i = 0; i < 6; ++i) xg_tiling_{name}[group][i] = set ? cfg[i] : xg_tiling_default_{name}[group][i];")
+        src.append(f"  xg_tiling_set_{name}[group] = (uint8_t)set;")
         src.append("  return 0;")
         src.append("}")
         src.append(f'extern "C" int xg_groups_{name}(void) {{ return {self.group_counter[0]}; }}')
@@ -618,6 +623,9 @@ class CudaGenerator:
         src.append(f"  if (group < 0 || group >= {max(self.group_counter[0], 1)}) return -1;")
         src.append(f"  for (int i = 0; i < 6; ++i) cfg[i] = xg_tiling_{name}[group][i];")
         src.append("  return 0;")
+        src.append("}")
+        src.append(f'extern "C" int xg_tiling_is_set_{name}(int group) {{')
+        src.append(f"  return group >= 0 && group < {max(self.group_counter[0], 1)} ? xg_tiling_set_{name}[group] : 0;")
         src.append("}")
         src.append(f'extern "C" int xg_mixed_{name}(int64_t every) {{ xg_mixed_every_{name} = every; return 0; }}')
         # error word of the persistent loops (1: a neighbour-tile wait gave up, the results

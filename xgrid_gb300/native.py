@@ -128,9 +128,10 @@ class NativeKernel:
         return 1 if err else 0
 
     # ---------------------------------------------------------------- tuning
-    def set_tiling(self, group: int, tiling: tuple) -> None:
-        """(tz, ty, tx, block.x, block.y, block.z) for one launch group."""
-        arr = (ctypes.c_int32 * 6)(*tiling)
+    def set_tiling(self, group: int, tiling: tuple | None) -> None:
+        """(tz, ty, tx, block.x, block.y, block.z) for one launch group; None: untuned, the
+        launch rules choose (strips, tile counts by the grid's extents)."""
+        arr = (ctypes.c_int32 * 6)(*(tiling or (0,) * 6))
         self.config_fn(group, arr, -1)
         runtime.load().xg_graph_clear(self.fn_ptr)
 
@@ -381,6 +382,10 @@ class NativeKernel:
         getter = getattr(self.lib.dylib, f"xg_get_tiling_{self.module.name}")
         getter(ctypes.c_int(group), arr)
         return tuple(arr)
+
+    def tiling_is_set(self, group: int) -> bool:
+        """Whether ``set_tiling`` fixed the group's tiling."""
+        return bool(getattr(self.lib.dylib, f"xg_tiling_is_set_{self.module.name}")(ctypes.c_int(group)))
 
 
 # steps per launch, tile rows, tile columns, CTA shape of the temporally blocked batched path
