@@ -1232,17 +1232,17 @@ def zstage_frame(kname: str, ptype: str, T: str, srcs: list, loads: list, outs: 
 
 
 def zstage_launch(kname: str, T: str, nb: int, ind: str, aligned: list, before: list, after: list,
-                  only_aligned: bool = False, nacc: int = 0) -> list:
+                  unaligned: str = "1", nacc: int = 0) -> list:
     """Host lines launching ``kname`` (a ``zstage_frame`` kernel) with parameters
     ``p`` on stream ``s`` when its shared memory fits; ``aligned``: the pointers
     (sources and destinations) that must be 16-byte aligned for 16-byte copies;
     ``before`` / ``after`` run around the launch, which ends with ``return 0``.
-    Falls through otherwise (with ``only_aligned`` also where rows are unaligned)."""
+    Falls through otherwise, and where rows are unaligned and ``unaligned`` is 0."""
     g = zstage_geometry(T, nb, nacc)
     ty, tx = ZSTAGE_TILE
     al = " && ".join(f"((uintptr_t)({a}) & 15) == 0" for a in aligned) or "1"
     # (vec, index type) of the instantiations; a kernel of unaligned rows has no old values to stage
-    kinds = [(v, it) for v in ((1,) if only_aligned else (1, 0)) for it in ("int", "int64_t")]
+    kinds = [(v, it) for v in (1, 0) for it in ("int", "int64_t")]
     L = ["{",
          f"  const int vec = (p.X % {g['V']}) == 0 && {al};",
          f"  const size_t smem = vec ? {g['smem']} : {g['smem'] - g['acc']};",
@@ -1255,7 +1255,7 @@ def zstage_launch(kname: str, T: str, nb: int, ind: str, aligned: list, before: 
     L += ["  int zlen = 0;",
           "  int64_t nt = 0;",
           f"  XG_TRY(xg_zstage_chunks(p.Z, p.Y, p.X, {ty}, {tx}, &zlen, &nt));",
-          f"  if ({'vec && ' if only_aligned else ''}smem <= (size_t)avail[vec][small] && nt <= 0x7fffffffLL) {{"]
+          f"  if ((vec || {unaligned}) && smem <= (size_t)avail[vec][small] && nt <= 0x7fffffffLL) {{"]
     L += ["    " + b for b in before]
     for v, it in kinds:
         cond = f"{'' if v else '!'}vec && {'' if it == 'int' else '!'}small"
@@ -2036,7 +2036,11 @@ class SweepGroupEmitter:
         swap = [f"{{ void* t_ = G[{s.slot}].level[{s.level}]; G[{s.slot}].level[{s.level}] = "
                 f"G[{s.slot}].scratch; G[{s.slot}].scratch = t_; }}"] if s.implicit else []
         if zbufs:
-            # a grid without boundary cells takes the staged z-walk (every tile mask-free)
+            # a grid without boundary cells takes the staged z-walk (every tile mask-free).  Unaligned rows of
+            # an untuned sweep that has strips go to those, or on grids that strips refuse to the tile kernel
+            # (200 x 200 x 35 FP32 diffusion 12.3 us staged 20.5, 50 x 50 x 33 9.8 both); under a set tiling
+            # they stay staged (203 x 245 x 307: 69 us; tiles 73 to 286 by the tiling, 128 the default one;
+            # 100 x 101 x 103: 10.3 against 12 to 88)
             L += [f"  if (p.same && xg_zstage_{n}) {{",
                   "    int64_t nz = 0;",
                   f"    XG_TRY(xg_mask_nonzero(G[{s.slot}].mask, &nz));",
@@ -2047,7 +2051,7 @@ class SweepGroupEmitter:
                                [f"if (xg_hook_{n}) XG_TRY(xg_hook_{n}(xg_hook_ctx_{n}, {site}, G, "
                                 f"{len(self.gen.slots)}, s));", f"xg_prof_launch({site}, s);",
                                 f"++xg_zstage_launches_{n};"],
-                               [f"xg_prof_end({site}, s);"], only_aligned=splan is not None)
+                               [f"xg_prof_end({site}, s);"], f"xg_tiling_set_{n}[{gid}]" if splan else "1")
             L += ["  }"]
         if splan:
             L += [f"  if (const int shape = xgl_{n}_{gid}_strips(G)) {{"]
