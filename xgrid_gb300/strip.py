@@ -44,6 +44,11 @@ FILL = 60  # a strip shape applies where the grid's columns fill at least this s
 # 14.5, 64^3 14.4 against 10.3
 MIN_CELLS = {2: 1 << 21, 3: 1 << 17}
 MIN_CELLS_PHASES = {2: 1 << 20, 3: 1 << 19}
+# from three phases on their launches weigh more, on 2-D rows of whole 32-column tiles, which the fused
+# launch takes best: four constant walls at 1024^2 12.3 against 10.2 us, 1024 x 1536 12.3 against 10.4,
+# 2048^2 16.4 against 16.9; ragged rows 1150^2 12.3 against 14.4, 1500^2 14.3 against 17.9.  (3-D: four
+# walls 80 x 80 x 96 14.4 both, six 16.6 against 16.4, 128^3 18.5 against 20.8)
+MANY_PHASES, MIN_CELLS_MANY = 3, 1 << 21
 
 
 def plan(em, j: int):
@@ -258,7 +263,10 @@ def apply_lines(em, pl) -> list:
     n, gid = em.name, em.gid
     dim, bufs = pl
     s = em.g.sweeps[0]
-    floor = (MIN_CELLS if len(em.g.sweeps) == 1 else MIN_CELLS_PHASES)[dim]
+    phases = len(em.g.sweeps) - 1
+    floor = (MIN_CELLS_PHASES if phases else MIN_CELLS)[dim]
+    if dim == 2 and phases >= MANY_PHASES:
+        floor = f"(dom.x % 32 == 0 ? {MIN_CELLS_MANY} : {floor})"
     L = [f"static int xgl_{n}_{gid}_strips(const xg_grid* G) {{",
          f"  const xg_ext dom = xg_extent(&G[{s.slot}]);",
          f"  if (!xg_zstage_{n} || xg_tiling_set_{n}[{gid}] || dom.z * dom.y * dom.x < {floor}) return 0;"]
