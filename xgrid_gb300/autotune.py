@@ -118,21 +118,27 @@ def _time(fn) -> float:
 
 
 # ---------------------------------------------------------------- batched
-def batch_candidates(one_dim: bool) -> list:
-    """(depth, ty, tx, block) candidates of the batched path (depth 1: one step per launch)."""
+def batch_candidates(one_dim: bool, registers: bool = True) -> list:
+    """(depth, ty, tx, block) candidates of the batched path (depth 1: one step per launch), for
+    kernels on register blocks or (FP64 fields, wider stencils) in shared memory alone."""
     if one_dim:
         out = [(1, 1, 256, (256, 1, 1))]
         for d in (2, 4, 6, 8, 12):
             for tx in (512, 1024, 2048):
                 out.append((d, 1, tx - 2 * d, (256, 1, 1)))
         return out
-    # tiles whose halo fills a box of 64 or 128 rows and columns (register blocks), and tiles of
-    # the shared-memory kernel that FP64 fields and wider stencils take
+    # tiles whose halo fills a box of 64 or 128 rows and columns.  In shared memory low tiles too, which
+    # spread little work (20 FP64 problems of 40 to 150 cells a side: 11.8 us a step with 16 rows, 15.7
+    # without; 8 of 64 to 512 with 2-cell reach 24.4 against 28.9), and no boxes of 128 x 128, which FP64
+    # has no room for and FP32 never took
     out = [(1, 32, 64, (32, 8, 1))]
     for d in (2, 4, 6, 8, 12):
         h = 2 * d
-        out += [(d, ty - h, tx - h, (32, 8, 1)) for ty in (64, 128) for tx in (64, 128)]
+        out += [(d, ty - h, tx - h, (32, 8, 1)) for ty in (64, 128) for tx in (64, 128)
+                if registers or ty + tx < 256]
         out += [(d, 32, tx - h, (32, 8, 1)) for tx in (64, 128)]
+    if not registers:
+        out += [(d, 16, 64 - 2 * d, (32, 8, 1)) for d in (2, 3, 4, 6)]
     return out
 
 
@@ -152,7 +158,7 @@ def tune_batch(native, problems, candidates=None) -> tuple:
     if hit is not None:
         return (int(hit[0]), int(hit[1]), int(hit[2]), tuple(int(b) for b in hit[3]))
     one_dim = all(len(s[0]) == 1 for s in shapes)
-    cands = candidates if candidates is not None else batch_candidates(one_dim)
+    cands = candidates if candidates is not None else batch_candidates(one_dim, native.module.batch_registers)
     snap = Snapshot(grids)
     results = []
     try:

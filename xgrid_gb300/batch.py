@@ -26,7 +26,6 @@ from __future__ import annotations
 
 from . import analysis, ir
 
-DEPTH_MAX = 8
 # register-block kernel: rows per warp and resident CTAs (of 8 warps) per SM asked of ptxas, by
 # fields.  16 rows make boxes of 128 rows, less of them halo and fewer barriers per cell: 15.0 us
 # a step for 60 problems of 64 to 1024 cells a side against 16.7 with 8 rows and 64-row boxes,

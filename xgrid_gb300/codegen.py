@@ -149,6 +149,7 @@ class Module:
     implicit_slots: list     # grid slots that need a scratch buffer
     aux_per_cell: dict       # grid slot -> bytes per cell of the mixed-precision work area
     batch: bool              # the module exports the batched entry points
+    batch_registers: bool    # its batched time loops have the register-block kernel
     groups: int
     device_only: bool        # kernel has no grid arguments (body runs on the device)
     sweeps: list             # analysis.Sweep per grid assignment (for the oracle and tests)
@@ -590,12 +591,14 @@ class CudaGenerator:
         for gi in range(max(self.group_counter[0], 1)):
             src.append("  {" + ", ".join(str(v) for v in self.group_tiling.get(gi, DEFAULT_TILING[2])) + "},")
         src.append("};")
-        batch_host = None
+        batch_host, batch_registers = None, False
         from . import batch as batch_mod
         if (not device_only and batch_mod.qualifies(self) and len(self.group_emitters) == 1
                 and batch_mod.BatchEmitter.usable(self.group_emitters[0].g)):
             em = self.group_emitters[0]
-            dev, batch_host = batch_mod.BatchEmitter(self, em.g, em).emit(value_args)
+            batched = batch_mod.BatchEmitter(self, em.g, em)
+            dev, batch_host = batched.emit(value_args)
+            batch_registers = batched.reg_plan()
             self.device_chunks.extend(dev)
         src.extend(self.device_chunks)
         src.extend(self.host_chunks)
@@ -646,7 +649,7 @@ class CudaGenerator:
         if getattr(self.op, "noalloc", False):
             src.extend(self.noalloc_entry(name, entry, grid_args, implicit))
         return Module("\n".join(src) + "\n", name, entry, self.depth + 1, grid_args, value_args, order, rtype,
-                      implicit, dict(self.mixed_slots), batch_host is not None, self.group_counter[0], device_only,
+                      implicit, dict(self.mixed_slots), batch_host is not None, batch_registers, self.group_counter[0], device_only,
                       self.sweeps)
 
     def noalloc_entry(self, name, entry, grid_args, implicit) -> list[str]:
