@@ -312,7 +312,7 @@ class NativeKernel:
                 self.logger.dead(runtime.last_error())
             B["nblocks"][threads] = nb.value
         ba = BatchArgs(dev.data_ptr(), total, steps, 0, B["counters"].data_ptr(), nprob, 1 if self.op.tick else 0,
-                       1 if maxc < (1 << 31) - 1 else 0, B["nblocks"][threads], (ctypes.c_int32 * 3)(*block))
+                       self._small_index(maxc), B["nblocks"][threads], (ctypes.c_int32 * 3)(*block))
         rc = runtime.load().xg_call(B["fn"], None, 0, ctypes.cast(ctypes.byref(ba), ctypes.c_void_p),
                                     ctypes.sizeof(ba), None, 0, device.stream_handle(), 1 if self.use_graph else 0)
         if rc != 0:
@@ -327,6 +327,12 @@ class NativeKernel:
             from . import autotune
             memo[shapes] = autotune.tune_batch(self, problems)
         return memo[shapes]
+
+    @staticmethod
+    def _small_index(cells: int) -> int:
+        """Whether batched kernels index problems of at most ``cells`` cells in 32 bits (as
+        ``xg_small_index`` says for single calls)."""
+        return 1 if cells < (1 << 31) - 1 and not runtime.load().xg_wide_index_forced() else 0
 
     def _after_batch(self, grids, steps: int, depth: int) -> None:
         for g in grids:
@@ -370,7 +376,7 @@ class NativeKernel:
             B["counters"] = device.alloc_bytes(steps * 8)
         fn = ctypes.cast(getattr(self.lib.dylib, f"xg_batch_tb_{self.module.name}"), ctypes.c_void_p).value
         ba = BatchTemporalArgs(dev.data_ptr(), total_tb, steps, B["counters"].data_ptr(), nprob,
-                               1 if maxc < (1 << 31) - 1 else 0, nb, depth, ty, tx, smem,
+                               self._small_index(maxc), nb, depth, ty, tx, smem,
                                (ctypes.c_int32 * 3)(*block))
         rc = runtime.load().xg_call(fn, None, 0, ctypes.cast(ctypes.byref(ba), ctypes.c_void_p),
                                     ctypes.sizeof(ba), None, 0, device.stream_handle(), 1 if self.use_graph else 0)
