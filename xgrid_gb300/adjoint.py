@@ -454,7 +454,7 @@ class AdjointGenerator:
             H += zstage_launch(f"xgk_{n}_adjoint_zs", T, len(bufs), "  ",
                                [bufs[k][0] for k in bufs] + ["p.lam_out"] + [f"p.g{sl}" for sl in slots_used
                                                                              if sl != self.slot],
-                               ["xg_prof_launch(-2, s);"], ["xg_prof_end(-2, s);"],
+                               ["xg_prof_launch(-3, s);"], ["xg_prof_end(-3, s);"],
                                nacc=sum(1 for _, _, _, add in zo if add))
         tz, ty, tx, bx, by = ZWALK_TILE if zwalk else (2, 16, 32, 32, 8)
         H += [f"  p.tz = {tz}; p.ty = {ty}; p.tx = {tx};",
