@@ -646,22 +646,31 @@ __device__ __forceinline__ void xg_tile_done(unsigned* flags, int64_t t, unsigne
 }
 
 // Cycles per iteration of a launch of th iterations on nb boxes of r core rows and w
-// columns, per_sm of them resident per SM: the boxes of the busiest SM share its FP64
-// pipe (half a cycle per cell and operation), a box alone takes its own latency, and a launch costs a ramp,
-// the staging and the write-back of every round of boxes.  The constants are fitted to
-// cavity steps (us, against 3 iterations in boxes that minimise cells per CTA slot):
-// 129^2 144 -> 109, 257^2 165 -> 151, 513^2 270 -> 269, 700^2 739 -> 682, 1025^2 722 -> 698,
-// 1200^2 1786 -> 1703, 1500^2 2564 -> 2472.
+// columns, per_sm of them resident per SM.  A launch costs a ramp, and the staging and
+// write-back of every box of the busiest SM; an iteration its barriers, and the larger of
+// the warps' latency and the SM's work: half a cycle per cell and FP64 operation (a warp's 32
+// columns cost the same with halo lanes off), the loop around cells that no later iteration
+// needs, and half a cycle more per cell of a box that has its SM to itself (one CTA does not fill
+// the pipe while its loads and barriers are under way), as the odd box of the last round and
+// every box too large for two to fit.  Three boxes on SMs that hold two end uneven: the last
+// ones go in pairs to the SMs that finish first.  The constants are fitted to 737 times of
+// 11 grid sizes by up to 24 shapes (four constant walls, 33^2 to 2500^2, FP64 with 4 and 5
+// operations and FP32; RMS error 3 %).  50 iterations of 4 operations, us, against a model
+// without the lone box's cost: 257^2 118 -> 111, 513^2 211 -> 206, 800^2 433 -> 356,
+// 1025^2 528 -> 519, 1300^2 986 -> 832, 1500^2 1121 -> 1066, 1850^2 2078 -> 1573.
 enum { XG_CYCLES_PER_US = 2070 };  // at the maximum SM clock
 static inline double xg_boxes_cost(int64_t nb, int sms, int per_sm, int nt, int ops, int r, int w, int th) {
   const int64_t most = (nb + sms - 1) / sms, rounds = (most + per_sm - 1) / per_sm;
-  double t = 6000;
+  const int64_t lone = per_sm == 1 ? most : most % 2;
+  const double area = (double)(r + 2 * th) * w, odd = 0.53 * lone + (per_sm > 1 && most == 3 ? 0.9 : 0);
+  double t = 6300 + 600 * rounds + 1.2 * most * area;
   for (int k = 1; k <= th; ++k) {
-    const double cells = (double)(r + 2 * th - 2 * k) * w;  // a warp's 32 columns cost the same with halo lanes off
-    const double pipe = most * cells * (0.6 * ops + 0.2), own = rounds * (700 + ceil(cells / nt) * 800);
-    t += pipe > own ? pipe : own;
+    const double cells = (double)(r + 2 * th - 2 * k) * w;
+    const double work = cells * (most * (0.425 * ops + 0.15) + odd) + 0.5 * most * (area - cells);
+    const double own = rounds * ceil(cells / nt) * 650;
+    t += 1000 * rounds + (work > own ? work : own);
   }
-  return (t + 2500 * rounds) / th;
+  return t / th;
 }
 
 // The core rows, box width and depth (t0 to t1 iterations) of boxes on a Y x X grid with the
