@@ -1471,9 +1471,11 @@ class SweepGroupEmitter:
     def tile_blocks(self) -> int:
         """Resident CTAs per SM of the group's tile kernel (the register z-walk keeps
         several planes in registers)."""
-        mains = [j for j, s in enumerate(self.g.sweeps) if s.is_main]
-        alone = len(self.g.sweeps) == 1 and len(mains) == 1
-        return ZWALK_BLOCKS if alone and self.zmarch_ok(mains, []) else self.min_blocks()
+        return ZWALK_BLOCKS if self.walks() else self.min_blocks()
+
+    def walks(self) -> bool:
+        """Whether the group's tile kernel is the register z-walk."""
+        return len(self.g.sweeps) == 1 and self.g.sweeps[0].is_main and self.zmarch_ok([0], [])
 
     def strip_plan(self):
         """Strip plan (``strip.plan``) of the group's main sweep when it is the only one
@@ -1936,7 +1938,7 @@ class SweepGroupEmitter:
             return [f"{indent}const int32_t* tl = xg_tiling_{n}[{gid}];"]
         return [f"{indent}int32_t tl_[6];",
                 f"{indent}const int32_t* tl = xg_tiling_for(xg_tiling_{n}[{gid}], xg_tiling_set_{n}[{gid}], "
-                f"&G[{slot}], {self.tile_blocks()}, tl_);",
+                f"&G[{slot}], {self.tile_blocks()}, {int(self.walks())}, tl_);",
                 f"{indent}if (!tl) return -1;"]
 
     def fill_params(self, tag: str, sweeps, dom_slot: int, single=None, indent: str = "  ",
