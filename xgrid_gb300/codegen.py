@@ -1463,10 +1463,13 @@ class SweepGroupEmitter:
         with 2 CTAs, 1290 with 4)."""
         if not self.wide():
             return 6
-        ops = sum(isinstance(e, ir.Binary) and not e.operator.is_compare() and not e.operator.is_logic()
-                  and has_stencil(e) and self.gen.ctype(e) == "double"
-                  for s in self.g.sweeps if s.is_main for e in ir.walk(s.stmt.value))
-        return 2 if ops >= FP64_HEAVY else BLOCKS_WIDE
+        return 2 if self.fp64_ops() >= FP64_HEAVY else BLOCKS_WIDE
+
+    def fp64_ops(self) -> int:
+        """FP64 operations per cell of the group's main sweeps."""
+        return sum(isinstance(e, ir.Binary) and not e.operator.is_compare() and not e.operator.is_logic()
+                   and has_stencil(e) and self.gen.ctype(e) == "double"
+                   for s in self.g.sweeps if s.is_main for e in ir.walk(s.stmt.value))
 
     def tile_blocks(self) -> int:
         """Resident CTAs per SM of the group's tile kernel (the register z-walk keeps

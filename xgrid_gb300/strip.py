@@ -38,6 +38,15 @@ WARPS = 4              # warps per CTA
 # diffusion 56 us (4 x 1: 64, 1 x 4: 66).
 SHAPE = {(2, 1): [(4, 1, 2, 6)], (2, 2): [(2, 1, 2, 6)], (3, 1): [(8, 1, 1, 4), (2, 2, 1, 6)], (3, 2): [(2, 2, 1, 4)]}
 FILL = 60  # a strip shape applies where the grid's columns fill at least this share (%) of its lanes
+# Sweeps that compute in FP64 (a Python literal is a double) are bound by the FP64 pipe, which strips
+# with idle lanes, or few of them, keep waiting.  2-D: narrow strips, but wide ones where they are full
+# and no mask is read (us, 128 against 64 columns: heat with walls 4097^2 206 and 199, 8192^2 757 and 750,
+# 1300^2 30.8 and 28.7; without 1500^2 34.9 and 30.8, 6000^2 406 and 411).  3-D, where the tile kernel
+# is no z-walk: strips only for ragged rows on 64 planes and more (tiles and strips, us: 384^3 755 and 922,
+# 256^3 232 and 246, 80 x 80 x 96 15.4 and 25.6, 24 x 1000 x 200 77 and 88, 9 x 60 x 1001 16.4 and 27.1;
+# but 203 x 201 x 205 139 and 129, 100 x 101 x 103 30.8 and 27.9).
+SHAPE_FP64_2D, FILL_FP64 = (2, 1, 2, 6), 99
+MIN_PLANES_FP64 = 64
 # smallest grids (cells), by dimension, without and with boundary phases (launches of their own
 # then): 2-D transport 2048^2 11.0 against 13.8 us on tiles, 1000^2 10.3 against 9.3; 3-D
 # diffusion 100^3 10.0 against 12.5; walls 2-D 1024^2 8.4 against 9.0, 3-D 80^3 13.6 against
@@ -79,10 +88,19 @@ def plan(em, j: int):
     return min(dims), bufs
 
 
+def shapes(em, pl) -> list:
+    """(strip shape, least fill) in the order of choice."""
+    dim, bufs = pl
+    out = [(s, FILL) for s in SHAPE[(dim, len(bufs))]]
+    if dim == 2 and len(bufs) == 1 and em.fp64_ops():
+        wide = [(out[0][0], FILL_FP64)] if len(em.g.sweeps) == 1 else []
+        out = wide + [(SHAPE_FP64_2D, FILL)]
+    return out
+
+
 def kernels(em, tag: str, j: int, pl) -> list:
     """One kernel per strip shape."""
-    dim, bufs = pl
-    return [_kernel(em, tag, j, pl, v, shape) for v, shape in enumerate(SHAPE[(dim, len(bufs))])]
+    return [_kernel(em, tag, j, pl, v, shape) for v, (shape, _) in enumerate(shapes(em, pl))]
 
 
 def _kernel(em, tag: str, j: int, pl, variant: int, shape: tuple) -> str:
@@ -272,9 +290,11 @@ def apply_lines(em, pl) -> list:
          f"  if (!xg_zstage_{n} || xg_tiling_set_{n}[{gid}] || dom.z * dom.y * dom.x < {floor}) return 0;"]
     L += [f"  if (!xg_same_ext(xg_extent(&G[{slot}]), dom)) return 0;"
           for slot in em.slots_used(em.g.sweeps) if slot != s.slot]
-    for v, (J, R, _, _) in enumerate(SHAPE[(dim, len(bufs))]):
+    if dim == 3 and em.fp64_ops() and not em.walks():
+        L.append(f"  if (dom.x % 32 == 0 || dom.z < {MIN_PLANES_FP64}) return 0;")
+    for v, ((J, R, _, _), fill) in enumerate(shapes(em, pl)):
         rows = f" && dom.y > {R}" if dim == 3 else ""  # a strip's rows reach at most one period beyond the grid
-        L.append(f"  if (100 * dom.x >= {FILL} * {32 * J} * ((dom.x + {32 * J - 1}) / {32 * J}){rows}) return {v + 1};")
+        L.append(f"  if (100 * dom.x >= {fill} * {32 * J} * ((dom.x + {32 * J - 1}) / {32 * J}){rows}) return {v + 1};")
     return L + ["  return 0;", "}"]
 
 
@@ -283,7 +303,7 @@ def launch(em, tag: str, pl, site: int, mask: str, ind: str) -> list:
     run the sweep on strips; the caller closes the two blocks that stay open."""
     n, gid = em.name, em.gid
     dim, bufs = pl
-    shapes = SHAPE[(dim, len(bufs))]
+    kinds = [shape for shape, _ in shapes(em, pl)]
     kname = f"xgk_{n}_{gid}_{tag}_rs"
     a, y = ("p.Z", "p.Y") if dim == 3 else ("p.Y", "1")
     pick = lambda xs: " : ".join(f"shape == {v + 1} ? {x}" for v, x in enumerate(xs)) + " : 0"
@@ -291,8 +311,8 @@ def launch(em, tag: str, pl, site: int, mask: str, ind: str) -> list:
          "  int alen = 0;",
          "  int64_t nsx = 0, nsy = 0, nw = 0, nz = 0;",
          "  const uint32_t* bits = NULL;",
-         f"  XG_TRY(xg_strip_chunks({a}, {y}, p.X, {pick([32 * v[0] for v in shapes])}, {pick([v[1] for v in shapes])}, "
-         f"{pick([WARPS * v[3] for v in shapes])}, &alen, &nsx, &nsy, &nw));",
+         f"  XG_TRY(xg_strip_chunks({a}, {y}, p.X, {pick([32 * v[0] for v in kinds])}, {pick([v[1] for v in kinds])}, "
+         f"{pick([WARPS * v[3] for v in kinds])}, &alen, &nsx, &nsy, &nw));",
          f"  XG_TRY(xg_mask_nonzero({mask}, &nz));",
          f"  if (nz != 0) XG_TRY(xg_mask_bits({mask}, &bits));",
          "  if (nw <= 0x3fffffffLL) {",
@@ -301,7 +321,7 @@ def launch(em, tag: str, pl, site: int, mask: str, ind: str) -> list:
          f"    const unsigned nb = (unsigned)((nw + {WARPS - 1}) / {WARPS});",
          "    const bool small = xg_small_index(p.Z, p.Y, p.X);"]
     first = True
-    for v in range(len(shapes)):
+    for v in range(len(kinds)):
         for it, c in (("int", "small"), ("int64_t", "!small")):
             for m, cm in (("false", "nz == 0"), ("true", "nz != 0")):
                 L.append(f"    {'' if first else 'else '}if (shape == {v + 1} && {c} && {cm}) {kname}{v}<{it}, {m}>"
