@@ -455,7 +455,7 @@ class AdjointGenerator:
                                [bufs[k][0] for k in bufs] + ["p.lam_out"] + [f"p.g{sl}" for sl in slots_used
                                                                              if sl != self.slot],
                                ["xg_prof_launch(-3, s);"], ["xg_prof_end(-3, s);"],
-                               nacc=sum(1 for _, _, _, add in zo if add))
+                               nacc=sum(1 for _, _, _, add in zo if add), ops=em.fp64_ops() if em.wide() else 0)
         tz, ty, tx, bx, by = ZWALK_TILE if zwalk else (2, 16, 32, 32, 8)
         H += [f"  p.tz = {tz}; p.ty = {ty}; p.tx = {tx};",
               "  p.ntz = xg_tiles_along(p.Z, p.tz); p.nty = xg_tiles_along(p.Y, p.ty); p.ntx = xg_tiles_along(p.X, p.tx);",

@@ -61,6 +61,9 @@ ZSTAGE_AHEAD = 1
 ZSTAGE_AHEAD_WIDE = 1  # with three or more staged buffers (three CTAs per SM still fit)
 ZSTAGE_MAX_BLOCKS = 3
 ZSTAGE_ONE_BARRIER = True
+# FP64 operations per cell from which the pipe bounds a plane and chunks follow xg_zstage_length_fp64:
+# 13 (three grids) 128^3 76 -> 68 us, 25 111 -> 96; but 7 (one grid, six neighbours) 200^3 135 -> 165
+ZSTAGE_FP64_OPS = 12
 
 # (tz, ty, tx, block.x, block.y, block.z) per grid dimensionality
 DEFAULT_TILING = {1: (1, 1, 1024, 256, 1, 1), 2: (1, 64, 32, 32, 8, 1), 3: (64, 4, 64, 64, 4, 1)}
@@ -1235,12 +1238,13 @@ def zstage_frame(kname: str, ptype: str, T: str, srcs: list, loads: list, outs: 
 
 
 def zstage_launch(kname: str, T: str, nb: int, ind: str, aligned: list, before: list, after: list,
-                  unaligned: str = "1", nacc: int = 0) -> list:
+                  unaligned: str = "1", nacc: int = 0, ops: int = 0) -> list:
     """Host lines launching ``kname`` (a ``zstage_frame`` kernel) with parameters
     ``p`` on stream ``s`` when its shared memory fits; ``aligned``: the pointers
     (sources and destinations) that must be 16-byte aligned for 16-byte copies;
     ``before`` / ``after`` run around the launch, which ends with ``return 0``.
-    Falls through otherwise, and where rows are unaligned and ``unaligned`` is 0."""
+    Falls through otherwise, and where rows are unaligned and ``unaligned`` is 0.  ``ops``:
+    FP64 operations per cell of the sweep."""
     g = zstage_geometry(T, nb, nacc)
     ty, tx = ZSTAGE_TILE
     al = " && ".join(f"((uintptr_t)({a}) & 15) == 0" for a in aligned) or "1"
@@ -1257,7 +1261,7 @@ def zstage_launch(kname: str, T: str, nb: int, ind: str, aligned: list, before: 
                  f"XG_TRY(xg_smem_optin({kname}<{it}, {'true' if v else 'false'}>, &avail[vec][small]));")
     L += ["  int zlen = 0;",
           "  int64_t nt = 0;",
-          f"  XG_TRY(xg_zstage_chunks(p.Z, p.Y, p.X, {ty}, {tx}, &zlen, &nt));",
+          f"  XG_TRY(xg_zstage_chunks(p.Z, p.Y, p.X, {ty}, {tx}, {int(ops >= ZSTAGE_FP64_OPS)}, &zlen, &nt));",
           f"  if ((vec || {unaligned}) && smem <= (size_t)avail[vec][small] && nt <= 0x7fffffffLL) {{"]
     L += ["    " + b for b in before]
     for v, it in kinds:
@@ -2059,7 +2063,8 @@ class SweepGroupEmitter:
                                [f"if (xg_hook_{n}) XG_TRY(xg_hook_{n}(xg_hook_ctx_{n}, {site}, G, "
                                 f"{len(self.gen.slots)}, s));", f"xg_prof_launch({site}, s);",
                                 f"++xg_zstage_launches_{n};"],
-                               [f"xg_prof_end({site}, s);"], f"xg_tiling_set_{n}[{gid}]" if splan else "1")
+                               [f"xg_prof_end({site}, s);"], f"xg_tiling_set_{n}[{gid}]" if splan else "1",
+                               ops=self.fp64_ops() if self.wide() else 0)
             L += ["  }"]
         if splan:
             L += [f"  if (const int shape = xgl_{n}_{gid}_strips(G)) {{"]

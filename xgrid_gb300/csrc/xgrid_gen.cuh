@@ -865,10 +865,22 @@ static inline int64_t xg_zstage_length(int64_t Z, int64_t ncb, int sms) {
   });
   return (Z + n - 1) / n;
 }
-static inline int xg_zstage_chunks(int64_t Z, int64_t Y, int64_t X, int ty, int tx, int* zlen, int64_t* nt) {
+// FP64 sweeps of many operations (`wide`): the pipe, not the copies, bounds a plane, so that a CTA alone on its SM loses
+// nothing and what counts is the rows of the busiest SM: (rounds + 1/2) * (planes per chunk + 3),
+// where a block of fewer rows (the last along y) is that much less work.  At least 4 planes.
+// Adjoint step and forward step of variable-coefficient diffusion, us, against the rule of FP32:
+// 256 x 64 x 100 283 -> 246 and 113 -> 111, 203 x 201 x 205 1376 -> 1264 and 551 -> 451, 128^3 279 ->
+// 246 and 111 -> 98, 64^3 88 -> 49 and 72 -> 41, 256^3 1871 and 723 both.
+static inline int64_t xg_zstage_length_fp64(int64_t Z, int64_t rows, int64_t slots) {
+  const int64_t n = xg_best_parts(Z, rows, slots, 1, Z / 4 > 1 ? Z / 4 : 1,
+                                  [](int64_t rounds, int64_t len) { return (2 * rounds + 1) * (len + 3); });
+  return (Z + n - 1) / n;
+}
+static inline int xg_zstage_chunks(int64_t Z, int64_t Y, int64_t X, int ty, int tx, int wide, int* zlen, int64_t* nt) {
   int sms = 0;
   XG_TRY(xg_sm_count(&sms));
-  const int64_t ncb = ((X + tx - 1) / tx) * ((Y + ty - 1) / ty), len = xg_zstage_length(Z, ncb, sms);
+  const int64_t nx = (X + tx - 1) / tx, ncb = nx * ((Y + ty - 1) / ty);
+  const int64_t len = wide ? xg_zstage_length_fp64(Z, nx * Y, (int64_t)sms * ty) : xg_zstage_length(Z, ncb, sms);
   *zlen = (int)len;
   *nt = ncb * ((Z + len - 1) / len);
   return 0;
