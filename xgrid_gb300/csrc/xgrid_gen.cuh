@@ -691,22 +691,23 @@ __device__ __forceinline__ void xg_tile_done(unsigned* flags, int64_t t, unsigne
 // needs, and half a cycle more per cell of a box that has its SM to itself (one CTA does not fill
 // the pipe while its loads and barriers are under way), as the odd box of the last round and
 // every box too large for two to fit.  Three boxes on SMs that hold two end uneven: the last
-// ones go in pairs to the SMs that finish first.  The constants are fitted to 737 times of
-// 11 grid sizes by up to 24 shapes (four constant walls, 33^2 to 2500^2, FP64 with 4 and 5
-// operations and FP32; RMS error 3 %).  50 iterations of 4 operations, us, against a model
-// without the lone box's cost: 257^2 118 -> 111, 513^2 211 -> 206, 800^2 433 -> 356,
-// 1025^2 528 -> 519, 1300^2 986 -> 832, 1500^2 1121 -> 1066, 1850^2 2078 -> 1573.
+// ones go in pairs to the SMs that finish first.  The constants are fitted to 1282 times of
+// 30 grid sizes by up to 24 shapes (four walls, 33^2 to 2500^2, FP32 and FP64 with 4, 5 and 9
+// operations; the shape picked is 2 % from the best one measured in the mean).  50 iterations
+// of 4 operations, us, against a model without the lone box's cost: 257^2 118 -> 111, 513^2
+// 211 -> 206, 800^2 433 -> 351, 1025^2 528 -> 519, 1300^2 986 -> 839, 1500^2 1121 -> 1066,
+// 1850^2 2078 -> 1573; of 9 operations 1300^2 1912 -> 1615, 1500^2 2023 both.
 enum { XG_CYCLES_PER_US = 2070 };  // at the maximum SM clock
 static inline double xg_boxes_cost(int64_t nb, int sms, int per_sm, int nt, int ops, int r, int w, int th) {
   const int64_t most = (nb + sms - 1) / sms, rounds = (most + per_sm - 1) / per_sm;
   const int64_t lone = per_sm == 1 ? most : most % 2;
-  const double area = (double)(r + 2 * th) * w, odd = 0.53 * lone + (per_sm > 1 && most == 3 ? 0.9 : 0);
-  double t = 6300 + 600 * rounds + 1.2 * most * area;
+  const double area = (double)(r + 2 * th) * w, odd = lone * (0.28 + 0.045 * ops) + (per_sm > 1 && most == 3 ? 0.85 : 0);
+  double t = 5700 + 1200 * rounds + 0.85 * most * area;
   for (int k = 1; k <= th; ++k) {
     const double cells = (double)(r + 2 * th - 2 * k) * w;
-    const double work = cells * (most * (0.425 * ops + 0.15) + odd) + 0.5 * most * (area - cells);
-    const double own = rounds * ceil(cells / nt) * 650;
-    t += 1000 * rounds + (work > own ? work : own);
+    const double work = cells * (most * (0.44 * ops + 0.2) + odd) + 0.18 * most * (area - cells);
+    const double own = rounds * (270 + ceil(cells / nt) * 650);
+    t += 1200 * rounds + (work > own ? work : own);
   }
   return t / th;
 }
