@@ -287,7 +287,8 @@ def apply_lines(em, pl) -> list:
         floor = f"(dom.x % 32 == 0 ? {MIN_CELLS_MANY} : {floor})"
     L = [f"static int xgl_{n}_{gid}_strips(const xg_grid* G) {{",
          f"  const xg_ext dom = xg_extent(&G[{s.slot}]);",
-         f"  if (!xg_zstage_{n} || xg_tiling_set_{n}[{gid}] || dom.z * dom.y * dom.x < {floor}) return 0;"]
+         f"  if (!xg_zstage_{n} || xg_tiling_set_{n}[{gid}] || dom.z * dom.y * dom.x < {floor}) return 0;",
+         "  if (dom.x > 0x3fffffffLL) return 0;  // a strip's columns and their neighbours are int"]
     L += [f"  if (!xg_same_ext(xg_extent(&G[{slot}]), dom)) return 0;"
           for slot in em.slots_used(em.g.sweeps) if slot != s.slot]
     if dim == 3 and em.fp64_ops() and not em.walks():
