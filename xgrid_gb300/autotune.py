@@ -120,7 +120,7 @@ def _time(fn) -> float:
 # ---------------------------------------------------------------- batched
 def batch_candidates(one_dim: bool, registers: bool = True) -> list:
     """(depth, ty, tx, block) candidates of the batched path (depth 1: one step per launch), for
-    kernels on register blocks or (FP64 fields, wider stencils) in shared memory alone."""
+    kernels on register blocks or (FP64 fields or arithmetic, wider stencils) in shared memory alone."""
     if one_dim:
         out = [(1, 1, 256, (256, 1, 1))]
         for d in (2, 4, 6, 8, 12):

@@ -87,11 +87,16 @@ class BatchEmitter:
         return ry, rx
 
     def reg_plan(self) -> bool:
-        """Whether the temporal steps can run on register blocks (``emit_reg``): FP32
-        fields on 2-D grids, every load within one cell on each axis."""
+        """Whether the temporal steps run on register blocks (``emit_reg``): FP32
+        fields on 2-D grids, every load within one cell on each axis, no FP64 operation
+        (a Python literal is a double): the FP64 pipe bounds those, and the blocks compute
+        every cell of a box of 64 or 128 rows in every step (tuned, us a step, blocks and
+        shared memory: one FP64 operation a cell, 60 problems of 64 to 1024 cells a side 57.4
+        and 52.1, 8 of 64 to 512 7.9 and 6.6; 9 points with three literals 157 and 145, 21.1
+        and 12.9; 20 of 40 to 150 21.5 and 12.5)."""
         gen, g = self.gen, self.g
         r = self.tb_plan()
-        if r is None or max(r) > 1:
+        if r is None or max(r) > 1 or self.e.fp64_ops():
             return False
         for s in g.sweeps:
             t = gen.defn.signature.arguments[self.e.arg_index(s.slot)][1]
