@@ -38,8 +38,9 @@ REPEATS = 2
 # A batched call of TUNE_STEPS steps that is shorter than SHORT_MS is bound by the host's launches, whose
 # noise used to pick the candidate: 8 problems of 64 to 512 cells a side 78.5 us a call of 50 steps on the
 # best one, 84 to 89 in two of six tunings.  Candidates within NEAR of the best are then timed again over
-# LONG_STEPS steps.
-SHORT_MS, NEAR, LONG_STEPS = 0.5, 1.4, 8 * TUNE_STEPS
+# LONG_STEPS steps.  (Host and launches of such a call take 0.08 ms; longer calls say enough by themselves:
+# 60 problems of 64 to 1024 cells a side, 0.35 ms, 1409 us a call of 96 steps, and 1441 by a second look.)
+SHORT_MS, NEAR, LONG_STEPS = 0.2, 1.4, 8 * TUNE_STEPS
 
 
 # ------------------------------------------------------------------ cache
