@@ -686,12 +686,12 @@ __device__ __forceinline__ void xg_tile_done(unsigned* flags, int64_t t, unsigne
 // Cycles per iteration of a launch of th iterations on nb boxes of r core rows and w
 // columns, per_sm of them resident per SM.  A launch costs a ramp, and the staging and
 // write-back of every box of the busiest SM; an iteration its barriers, and the larger of
-// the warps' latency and the SM's work: half a cycle per cell and FP64 operation (a warp's 32
+// the warps' latency and the SM's work: 0.44 cycles per cell and FP64 operation (a warp's 32
 // columns cost the same with halo lanes off), the loop around cells that no later iteration
-// needs, and half a cycle more per cell of a box that has its SM to itself (one CTA does not fill
-// the pipe while its loads and barriers are under way), as the odd box of the last round and
-// every box too large for two to fit.  Three boxes on SMs that hold two end uneven: the last
-// ones go in pairs to the SMs that finish first.  The constants are fitted to 1282 times of
+// needs, and 0.28 + 0.045 per operation more per cell of a box that has its SM to itself (one CTA
+// does not fill the pipe while its loads and barriers are under way), as the odd box of the last
+// round and every box too large for two to fit.  Three boxes on SMs that hold two end uneven: the
+// last ones go in pairs to the SMs that finish first.  The constants are fitted to 1282 times of
 // 30 grid sizes by up to 24 shapes (four walls, 33^2 to 2500^2, FP32 and FP64 with 4, 5 and 9
 // operations; the shape picked is 2 % from the best one measured in the mean).  50 iterations
 // of 4 operations, us, against a model without the lone box's cost: 257^2 118 -> 111, 513^2
